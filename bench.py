@@ -318,7 +318,9 @@ def kernel_name(st):
         return f"k_fft_fast<IN_ROW={st.get('in_row', 0)}>"
     if st["kind"] == "plane":
         return "k_fft_plane_cluster" if st.get("cluster") else "k_fft_plane_flow"
-    return "k_fft_pass" if st["kind"] == "pass" else f"k_bs/{st['kind']}"
+    if st["kind"] == "pass":
+        return "k_fft_mix" if st.get("radices") else "k_fft_direct"
+    return f"k_bs/{st['kind']}"
 
 
 def nd_norm_factor_c64(n):

@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1)
                 typename Cx<T>::type* const* src, typename Cx<T>::type* const* dst, int* done,
                 unsigned long long* ticket, int* err, int conj, double scale, unsigned spin_limit) {
   using C = typename Cx<T>::type;
+  constexpr int VW = sizeof(T) == 4 ? 2 : 1;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   C* sm = reinterpret_cast<C*>(smem_raw);
   __shared__ __align__(16) PassGeom sg;
@@ -175,7 +176,10 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1)
     tb.k2p = d.k2p;
     C* o = dst[d.transform];
     const C* in = (d.pass == 0) ? src[d.transform] : o;
-    generic_tile<T, 0, 0>(sg, in, o, tb, s_t - start[slot], sm);
+    if (sg.nst == 0)
+      direct_tile<T>(sg, in, o, tb, s_t - start[slot], sm);
+    else
+      mix_tile<T, VW, true>(sg, in, o, tb, s_t - start[slot], sm);
     __syncthreads();
     if (threadIdx.x == 0) {
       __threadfence();
@@ -341,6 +345,7 @@ int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, int 
     g.in_row = row ? 1 : 0;
     g.out_row = row ? 1 : 0;
     g.scale = 1.0;
+    geom_derive(g);
     const size_t smem = (size_t)L * g.pitch * es;
     float ms = 0;
     for (int rep = 0; rep < 4; ++rep) {
@@ -408,6 +413,7 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
     int transform, pass, last, prev;
   };
   std::vector<std::vector<HostSlot>> per_transform(b->count);
+  std::map<int64_t, RadixPlan> plans;  // by axis length
   size_t maxsmem = 0;
   const int64_t* dp = b->dims.data();
   for (int t = 0; t < b->count; ++t) {
@@ -426,7 +432,8 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
       for (int c = 0; c < a; ++c) O *= dims[c];
       HostSlot hs{};
       PassGeom& g = hs.g;
-      RadixPlan rp = radix_plan((int)L);
+      if (!plans.count(L)) plans[L] = radix_plan((int)L);
+      const RadixPlan& rp = plans[L];
       g.L = (int)L;
       g.nst = rp.n > 0 ? rp.n : 0;
       for (int s = 0; s < g.nst; ++s) g.rad[s] = rp.r[s];
@@ -454,6 +461,8 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
       int cap = 1;
       while (cap < g.ext[0] && cap < kBatchRowWMax) cap *= 2;
       W = std::max(1, std::min(W, cap));
+      // radix passes work on 16-byte chunks: two complex64 columns
+      if (g.nst > 0) W = std::max(W, sizeof(T) == 4 ? 2 : 1);
       g.W = W;
       g.logW = 0;
       while ((1 << g.logW) < W) ++g.logW;
@@ -463,6 +472,7 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
       g.in_row = row ? 1 : 0;
       g.out_row = row ? 1 : 0;
       g.scale = 1.0;
+      geom_derive(g);
       maxsmem = std::max(maxsmem, (size_t)L * g.pitch * es);
       if (!lens.count(L)) lens[L] = LenTab{alloc(es * L), alloc(2 * L), alloc(2 * L)};
       hs.L = L;
@@ -488,6 +498,7 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
       g.ntiles = n;
       g.in_row = g.out_row = 1;
       g.scale = 1.0;
+      geom_derive(g);
       if (!lens.count(1)) lens[1] = LenTab{alloc(es), alloc(2), alloc(2)};
       hs.L = 1;
       hs.transform = t;
@@ -585,7 +596,7 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
     BCUDA(cudaMalloc(&b->d_tslot, sizeof(int) * std::max<size_t>(ts.size(), 1)));
     if (!ts.empty()) BCUDA(cudaMemcpy(b->d_tslot, ts.data(), sizeof(int) * ts.size(), cudaMemcpyHostToDevice));
   }
-  b->smem = std::max<size_t>(maxsmem, 16);
+  b->smem = std::max<size_t>((maxsmem + 127) & ~size_t(127), 128);  // slots are permuted within 128 bytes
   BCUDA(cudaFuncSetAttribute(k_fft_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)std::max<size_t>(b->smem, 48 * 1024)));
   int dev = 0, sms = 148, per = 1;

@@ -4,7 +4,8 @@
 // w = exp(-2*pi*i/R), natural order in and out.  The backward transform is
 // obtained by the passes through conjugation at load and store, so only the
 // forward sign is compiled.  Radix 4/8/16 are built from radix-2/4 with the
-// Cooley-Tukey split n = n1 + N1*n2, k = N2*k1 + k2; odd primes use the
+// Cooley-Tukey split n = n1 + N1*n2, k = N2*k1 + k2, 9 from 3 x 3 the same way,
+// 6, 10 and 12 from their coprime factors without twiddles; odd primes use the
 // symmetric-pair form that needs (p-1)^2/2 real multiply-adds per component.
 #pragma once
 #include <cuda_runtime.h>
@@ -210,6 +211,61 @@ __device__ __forceinline__ void dft_odd(C* v) {
   v[0] = s0;
 }
 
+// 9 points as 3 x 3 (n = n1 + 3 n2, k = 3 k1 + k2): DFT3 over n2, twiddle
+// w9^{n1 k2}, DFT3 over n1
+template <typename C>
+__device__ __forceinline__ void dft9(C* v) {
+  C y[3][3];
+#pragma unroll
+  for (int n1 = 0; n1 < 3; ++n1) {
+    y[n1][0] = v[n1];
+    y[n1][1] = v[n1 + 3];
+    y[n1][2] = v[n1 + 6];
+    dft_odd<3>(y[n1]);
+  }
+  y[1][1] = ctw<9, 1>(y[1][1]);
+  y[1][2] = ctw<9, 2>(y[1][2]);
+  y[2][1] = ctw<9, 2>(y[2][1]);
+  y[2][2] = ctw<9, 4>(y[2][2]);
+#pragma unroll
+  for (int k2 = 0; k2 < 3; ++k2) {
+    C t[3] = {y[0][k2], y[1][k2], y[2][k2]};
+    dft_odd<3>(t);
+    v[k2] = t[0];
+    v[k2 + 3] = t[1];
+    v[k2 + 6] = t[2];
+  }
+}
+
+template <int R, typename C>
+__device__ __forceinline__ void dft(C* v);
+
+// R = A * B points with A, B coprime (prime-factor split): with
+// n = (B n1 + A n2) mod R, w_R^{nk} = w_A^{n1 k} w_B^{n2 k}, so X[k] is entry
+// (k mod A, k mod B) of the A x B two-dimensional DFT; no twiddles
+template <int A, int B, typename C>
+__device__ __forceinline__ void dft_coprime(C* v) {
+  constexpr int R = A * B;
+  C y[A][B];
+#pragma unroll
+  for (int n1 = 0; n1 < A; ++n1) {
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) y[n1][n2] = v[(B * n1 + A * n2) % R];
+    dft<B>(y[n1]);
+  }
+#pragma unroll
+  for (int k2 = 0; k2 < B; ++k2) {
+    C t[A];
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) t[n1] = y[n1][k2];
+    dft<A>(t);
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) y[n1][k2] = t[n1];
+  }
+#pragma unroll
+  for (int k = 0; k < R; ++k) v[k] = y[k % A][k % B];
+}
+
 template <int R, typename C>
 __device__ __forceinline__ void dft(C* v) {
   if constexpr (R == 1) {
@@ -223,6 +279,14 @@ __device__ __forceinline__ void dft(C* v) {
     dft16(v);
   } else if constexpr (R == 32) {
     dft32(v);
+  } else if constexpr (R == 6) {
+    dft_coprime<2, 3>(v);
+  } else if constexpr (R == 9) {
+    dft9(v);
+  } else if constexpr (R == 10) {
+    dft_coprime<2, 5>(v);
+  } else if constexpr (R == 12) {
+    dft_coprime<4, 3>(v);
   } else {
     static_assert(R == 3 || R == 5 || R == 7 || R == 11 || R == 13, "unsupported radix");
     dft_odd<R>(v);

@@ -126,17 +126,12 @@ struct FastTileAt {
 };
 template <int W>
 __device__ __forceinline__ FastTileAt fast_tile_at(const PassGeom& g, int64_t tile) {
-  const int64_t tw = tile % g.tiles_w;
-  int64_t rest = tile / g.tiles_w;
-  const int64_t i1 = rest % g.ext[1];
-  rest /= g.ext[1];
-  const int64_t i2 = rest % g.ext[2];
-  const int64_t i3 = rest / g.ext[2];
+  const TileIdx x = tile_idx(g, tile);
   FastTileAt a;
-  a.w0 = tw * W;
-  a.bin = a.w0 * g.sin[0] + i1 * g.sin[1] + i2 * g.sin[2] + i3 * g.sin[3];
-  a.bout = a.w0 + i1 * g.sout[1] + i2 * g.sout[2] + i3 * g.sout[3];
-  a.tconst = g.tw_dim == 1 ? i1 : (g.tw_dim == 2 ? i2 : (g.tw_dim == 3 ? i3 : 0));
+  a.w0 = x.tw * W;
+  a.bin = a.w0 * g.sin[0] + x.i1 * g.sin[1] + x.i2 * g.sin[2] + x.i3 * g.sin[3];
+  a.bout = a.w0 + x.i1 * g.sout[1] + x.i2 * g.sout[2] + x.i3 * g.sout[3];
+  a.tconst = g.tw_dim == 1 ? x.i1 : (g.tw_dim == 2 ? x.i2 : (g.tw_dim == 3 ? x.i3 : 0));
   return a;
 }
 

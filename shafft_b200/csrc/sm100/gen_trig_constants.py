@@ -9,7 +9,7 @@ from decimal import Decimal, getcontext
 
 getcontext().prec = 60
 PRIMES = [3, 5, 7, 11, 13]
-POW2 = [8, 16, 32]
+POW2 = [8, 9, 16, 32]  # and 9 = 3 * 3, whose butterfly needs twiddles too
 
 
 def pi():

@@ -1,120 +1,18 @@
-// Device kernels of the sm_100a C2C FFT backend.
+// Direct-DFT pass, element-wise kernels and table generation of the sm_100a
+// C2C FFT backend.
 //
-// k_fft_pass  -- one HBM pass: batched length-L DFTs on W-wide tiles.
-//   Phase 1: each thread loads the R inputs of a first-stage butterfly
-//            straight from HBM (coalesced: lanes walk b0 for column tiles or
-//            n for row tiles), applies input conjugation / four-step
-//            pre-twiddle, runs the radix-R butterfly in registers, applies
-//            the decimation-in-frequency twiddle and writes the R results to
-//            shared memory in place.
-//   Phase 2: the remaining radix stages run in shared memory, in place
-//            (Cooley-Tukey DIF; span shrinks by the stage radix).  The
-//            shared tile is [L][W] with an odd row pitch (W+1), so 16 lanes
-//            that share a row and differ in w never hit the same bank, and
-//            16 lanes that walk rows with a fixed w do not either.
-//   Phase 3: results are read back in digit-reversed order through a small
-//            permutation table and stored to HBM with the four-step
-//            post-twiddle, scale and output conjugation fused in.
-// The same source serves a runtime length (LS == 0) and compile-time
-// specialisations for the hot lengths, where all index arithmetic folds.
+// k_fft_direct -- one HBM pass of batched length-L DFTs on W-wide tiles for
+// lengths with a prime factor above 13: the tile is loaded in natural order
+// and every output is an O(L) sum, evaluated in pairs (direct_store).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "butterflies.cuh"
+#include "mix.cuh"
 #include "pass.h"
 
 namespace shafft_sm100 {
-
-template <typename C>
-__device__ __forceinline__ C tw_n(const PassTables<C>& tb, int shift, int64_t mask, int64_t m) {
-  C hi = tb.tw_hi[m >> shift];
-  C lo = tb.tw_lo[m & mask];
-  return cmul(hi, lo);
-}
-
-template <int R, typename C>
-__device__ __forceinline__ void stage_first(const PassGeom& g, const PassTables<C>& tb, const C* in,
-                                            C* sm, int L, int W, int logW, int pitch, int nst,
-                                            int wcount, int64_t bin, int64_t w0, int64_t tconst) {
-  const int m0 = L / R;
-  const int nbf = m0 << logW;
-  for (int b = threadIdx.x; b < nbf; b += kThreads) {
-    int w, j;
-    if (g.in_row) {
-      j = b % m0;
-      w = b / m0;
-    } else {
-      w = b & (W - 1);
-      j = b >> logW;
-    }
-    const bool valid = w < wcount;
-    const C* src = in + bin + (int64_t)w * g.sin[0];
-    C v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int n = j + r * m0;
-      C x = valid ? src[(int64_t)n * g.sn_in] : C{0, 0};
-      if (g.conj_in) x.y = -x.y;
-      if (g.tw_mode == TW_PRE) {
-        const int64_t t = (g.tw_dim == 0) ? (w0 + w) : tconst;
-        x = cmul(x, tw_n(tb, g.tw_shift, g.tw_mask, (int64_t)n * t));
-      }
-      v[r] = x;
-    }
-    dft<R>(v);
-    if (nst > 1 && j != 0) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], tb.twL[j * r]);
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) sm[(j + r * m0) * pitch + w] = v[r];
-  }
-}
-
-template <int R, typename C>
-__device__ __forceinline__ void stage_mid(const PassTables<C>& tb, C* sm, int L, int W, int logW,
-                                          int pitch, int span, int Ls) {
-  const int m = span / R;
-  const int nbf = (L / R) << logW;
-  for (int b = threadIdx.x; b < nbf; b += kThreads) {
-    const int w = b & (W - 1);
-    const int q = b >> logW;
-    const int blk = q / m;
-    const int j = q - blk * m;
-    const int base = blk * span + j;
-    C v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = sm[(base + r * m) * pitch + w];
-    dft<R>(v);
-    if (m > 1 && j != 0) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], tb.twL[j * r * Ls]);
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) sm[(base + r * m) * pitch + w] = v[r];
-  }
-}
-
-#define SHAFFT_RADIX_DISPATCH(RAD, CALL) \
-  switch (RAD) {                         \
-    case 2: CALL(2); break;              \
-    case 3: CALL(3); break;              \
-    case 4: CALL(4); break;              \
-    case 5: CALL(5); break;              \
-    case 7: CALL(7); break;              \
-    case 8: CALL(8); break;              \
-    case 11: CALL(11); break;            \
-    case 13: CALL(13); break;            \
-    case 16: CALL(16); break;            \
-    default: break;                      \
-  }
-
-__host__ __device__ constexpr int ilog2c(int x) {
-  int l = 0;
-  while ((1 << l) < x) ++l;
-  return l;
-}
 
 // One output of a direct-DFT tile, with the pass's fused post-twiddle,
 // scale and output conjugation.
@@ -208,136 +106,42 @@ __device__ __forceinline__ void direct_store(const PassGeom& g, const PassTables
   }
 }
 
-// One W-wide tile of a generic pass (runtime length and radix list; nst == 0
-// selects the direct DFT).  `sm` holds L * pitch elements.
-template <typename T, int LS, int WS>
-__device__ __forceinline__ void generic_tile(const PassGeom& g, const typename Cx<T>::type* in,
-                                             typename Cx<T>::type* out,
-                                             const PassTables<typename Cx<T>::type>& tb, int64_t tile,
-                                             typename Cx<T>::type* sm) {
+// One tile of a direct-DFT pass.  `sm` holds L * pitch elements.
+template <typename T>
+__device__ __forceinline__ void direct_tile(const PassGeom& g, const typename Cx<T>::type* in,
+                                            typename Cx<T>::type* out,
+                                            const PassTables<typename Cx<T>::type>& tb, int64_t tile,
+                                            typename Cx<T>::type* sm) {
   using C = typename Cx<T>::type;
-  constexpr RadixPlan P = radix_plan(LS > 0 ? LS : 1);
-  const int L = LS ? LS : g.L;
-  const int W = WS ? WS : g.W;
-  const int logW = WS ? ilog2c(WS) : g.logW;
-  const int pitch = g.pitch;  // generic_pitch(W, in_row), set by the planner
-  const int nst = LS ? P.n : g.nst;
-
-  int64_t rest = tile;
-  const int64_t tw = rest % g.tiles_w;
-  rest /= g.tiles_w;
-  const int64_t i1 = rest % g.ext[1];
-  rest /= g.ext[1];
-  const int64_t i2 = rest % g.ext[2];
-  const int64_t i3 = rest / g.ext[2];
-  const int64_t w0 = tw * W;
-  const int wcount = (int)((g.ext[0] - w0) < W ? (g.ext[0] - w0) : W);
-  const int64_t bin = w0 * g.sin[0] + i1 * g.sin[1] + i2 * g.sin[2] + i3 * g.sin[3];
-  const int64_t bout = w0 * g.sout[0] + i1 * g.sout[1] + i2 * g.sout[2] + i3 * g.sout[3];
-  const int64_t tconst = g.tw_dim == 1 ? i1 : (g.tw_dim == 2 ? i2 : (g.tw_dim == 3 ? i3 : 0));
-
-  if (!LS && nst == 0) {
-    // direct DFT: load the tile in natural order, then O(L) per output
-    const int total = L << logW;
-    for (int b = threadIdx.x; b < total; b += kThreads) {
-      int w, n;
-      if (g.in_row) {
-        n = b % L;
-        w = b / L;
-      } else {
-        w = b & (W - 1);
-        n = b >> logW;
-      }
-      C x = (w < wcount) ? in[bin + (int64_t)w * g.sin[0] + (int64_t)n * g.sn_in] : C{0, 0};
-      if (g.conj_in) x.y = -x.y;
-      if (g.tw_mode == TW_PRE) {
-        const int64_t t = (g.tw_dim == 0) ? (w0 + w) : tconst;
-        x = cmul(x, tw_n(tb, g.tw_shift, g.tw_mask, (int64_t)n * t));
-      }
-      sm[n * pitch + w] = x;
+  const int L = g.L, W = g.W;
+  const TileAt at = tile_at(g, tile);
+  const int total = L << g.logW;
+  for (int b = threadIdx.x; b < total; b += kThreads) {
+    int w, n;
+    if (g.in_row) {
+      n = b % L;
+      w = b / L;
+    } else {
+      w = b & (W - 1);
+      n = b >> g.logW;
     }
-    __syncthreads();
-    direct_store<T, C>(g, tb, sm, out, L, W, logW, pitch, wcount, bout, w0, tconst);
-    return;
-  }
-
-  // phase 1: load + first radix stage
-  {
-    const int r0 = LS ? P.r[0] : g.rad[0];
-#define SHAFFT_CALL_FIRST(R) \
-  stage_first<R, C>(g, tb, in, sm, L, W, logW, pitch, nst, wcount, bin, w0, tconst)
-    SHAFFT_RADIX_DISPATCH(r0, SHAFFT_CALL_FIRST)
-#undef SHAFFT_CALL_FIRST
+    C x = (w < at.wcount) ? in[at.bin + (int64_t)w * g.sin[0] + (int64_t)n * g.sn_in] : C{0, 0};
+    if (g.conj_in) x.y = -x.y;
+    sm[n * g.pitch + w] = x;
   }
   __syncthreads();
-  // phase 2: remaining stages in shared memory
-  {
-    int span = L;
-#pragma unroll
-    for (int s = 1; s < (LS ? P.n : kMaxStages); ++s) {
-      if (!LS && s >= nst) break;
-      span /= (LS ? P.r[s - 1] : g.rad[s - 1]);
-      const int Ls = L / span;
-      const int rs = LS ? P.r[s] : g.rad[s];
-#define SHAFFT_CALL_MID(R) stage_mid<R, C>(tb, sm, L, W, logW, pitch, span, Ls)
-      SHAFFT_RADIX_DISPATCH(rs, SHAFFT_CALL_MID)
-#undef SHAFFT_CALL_MID
-      __syncthreads();
-    }
-  }
-  // phase 3: digit-reversed read, fused twiddle/scale/conj, store
-  const int total = L << logW;
-  const T scale = (T)g.scale;
-  if (g.out_row) {
-    for (int b = threadIdx.x; b < total; b += kThreads) {
-      const int k = b % L, w = b / L;
-      if (w >= wcount) continue;
-      C x = sm[tb.k2p[k] * pitch + w];
-      if (g.tw_mode == TW_POST) {
-        const int64_t t = (g.tw_dim == 0) ? (w0 + w) : tconst;
-        x = cmul(x, tw_n(tb, g.tw_shift, g.tw_mask, (int64_t)k * t));
-      }
-      if (g.scale != 1.0) x = cscale(x, scale);
-      if (g.conj_out) x.y = -x.y;
-      out[bout + (int64_t)w * g.sout[0] + (int64_t)k * g.sk_out] = x;
-    }
-  } else {
-    // column output walked in natural k order: a thread keeps its column
-    // w = tid mod W (W divides kThreads) and visits k = k0, k0 + KS, ...
-    // (KS = kThreads / W), so the four-step twiddle w_N^{k t} is a running
-    // product by w_N^{KS t}, taken afresh from the table every 4 outputs
-    // (the table reads are scattered across the lanes)
-    const int KS = kThreads >> logW;
-    const int w = threadIdx.x & (W - 1);
-    const bool tw = g.tw_mode == TW_POST && w < wcount;
-    const int64_t t = (g.tw_dim == 0) ? (w0 + w) : tconst;
-    C tstep = C{1, 0}, tcur = C{1, 0};
-    if (tw && KS < L) tstep = tw_n(tb, g.tw_shift, g.tw_mask, (int64_t)KS * t);
-    int i = 0;
-    for (int b = threadIdx.x; b < total; b += kThreads, ++i) {
-      if (w >= wcount) continue;
-      const int k = b >> logW;
-      C x = sm[tb.k2p[k] * pitch + w];
-      if (tw) {
-        tcur = (i % 4 == 0) ? tw_n(tb, g.tw_shift, g.tw_mask, (int64_t)k * t) : cmul(tcur, tstep);
-        x = cmul(x, tcur);
-      }
-      if (g.scale != 1.0) x = cscale(x, scale);
-      if (g.conj_out) x.y = -x.y;
-      out[bout + (int64_t)w * g.sout[0] + (int64_t)k * g.sk_out] = x;
-    }
-  }
+  direct_store<T, C>(g, tb, sm, out, L, W, g.logW, g.pitch, at.wcount, at.bout, at.w0, at.tconst);
 }
 
-template <typename T, int LS, int WS>
+template <typename T>
 __global__ void __launch_bounds__(kThreads)
-    k_fft_pass(const __grid_constant__ PassGeom g, const typename Cx<T>::type* in,
-               typename Cx<T>::type* out, const __grid_constant__ PassTables<typename Cx<T>::type> tb) {
+    k_fft_direct(const __grid_constant__ PassGeom g, const typename Cx<T>::type* in,
+                 typename Cx<T>::type* out, const __grid_constant__ PassTables<typename Cx<T>::type> tb) {
   using C = typename Cx<T>::type;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   C* sm = reinterpret_cast<C*>(smem_raw);
   for (int64_t tile = blockIdx.x; tile < g.ntiles; tile += gridDim.x) {
-    generic_tile<T, LS, WS>(g, in, out, tb, tile, sm);
+    direct_tile<T>(g, in, out, tb, tile, sm);
     __syncthreads();
   }
 }

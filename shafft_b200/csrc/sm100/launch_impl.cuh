@@ -480,27 +480,36 @@ SHAFFT_DEFINE_PRECISION(double, SHAFFT_FAST_LIST_F64, SHAFFT_PLANE_LIST_F64)
 #undef TYPE_
 #endif
 
-// Compile-time instances of the generic pass (length, tile width): the radix
-// sequence and every index division fold into constants.  The lengths are
-// the factors of the 3^5*5^3*7^2 = 1,488,375 FFT1D plan (1215 * 1225) at the
-// tile widths its complex64 (4) and complex128 (2) plans use; measured on
-// B200 the complex64 transform drops from 0.108 to 0.099 ms fwd+bwd.
-#define SHAFFT_GENERIC_LIST(X) \
-  X(1215, 4)                   \
-  X(1225, 4)                   \
-  X(1215, 2)                   \
-  X(1225, 2)
+// Threads of a generic pass: the block size up to 256 that leaves the fewest
+// thread slots idle over the stages (ties to the larger block).
+static int mix_threads(const PassGeom& g, int nc) {
+  int best = 32;
+  double least = 1e30;
+  for (int nt = 32; nt <= kThreads; nt += 32) {
+    double slots = 0;
+    for (int s = 0; s < g.nst; ++s) {
+      const int nbf = g.L / g.rad[s] * nc;
+      const int rounds = (nbf + nt - 1) / nt;
+      // a block of few threads takes more rounds, each with its own latency
+      slots += (double)rounds * nt / nbf + 0.02 * rounds;
+    }
+    if (slots <= least) {
+      least = slots;
+      best = nt;
+    }
+  }
+  return best;
+}
 
 template <typename T>
 cudaError_t Launch<T>::init() {
-  cudaError_t e = cudaFuncSetAttribute(k_fft_pass<T, 0, 0>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-#define SHAFFT_ATTR_GENERIC(L_, W_)                                                          \
-  if (e == cudaSuccess)                                                                      \
-    e = cudaFuncSetAttribute(k_fft_pass<T, L_, W_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                             200 * 1024);
-  SHAFFT_GENERIC_LIST(SHAFFT_ATTR_GENERIC)
-#undef SHAFFT_ATTR_GENERIC
+  constexpr int kMaxSmem = 200 * 1024;
+  constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  constexpr int VW = sizeof(T) == 4 ? 2 : 1;
+  cudaError_t e = cudaFuncSetAttribute(k_fft_direct<T>, kAttr, kMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_fft_mix<T, 1, true>, kAttr, kMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_fft_mix<T, VW, true>, kAttr, kMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_fft_mix<T, VW, false>, kAttr, kMaxSmem);
   if (e != cudaSuccess) return e;
   return fast_attr_all<T>();
 }
@@ -526,15 +535,24 @@ cudaError_t Launch<T>::init_device() {
 template <typename T>
 cudaError_t Launch<T>::pass(const PassGeom& g, const C* in, C* out, const PassTables<C>& tb,
                             size_t smem, cudaStream_t s) {
-  const int64_t grid = std::min<int64_t>(g.ntiles, 148 * 64);
-#define SHAFFT_CASE_GENERIC(L_, W_)                                                    \
-  if (g.L == L_ && g.W == W_) {                                                        \
-    k_fft_pass<T, L_, W_><<<(unsigned)grid, kThreads, smem, s>>>(g, in, out, tb);      \
-    return cudaGetLastError();                                                         \
+  if (g.nst == 0) {
+    const int64_t grid = std::min<int64_t>(g.ntiles, 148 * 64);
+    k_fft_direct<T><<<(unsigned)grid, kThreads, smem, s>>>(g, in, out, tb);
+    return cudaGetLastError();
   }
-  SHAFFT_GENERIC_LIST(SHAFFT_CASE_GENERIC)
-#undef SHAFFT_CASE_GENERIC
-  k_fft_pass<T, 0, 0><<<(unsigned)grid, kThreads, smem, s>>>(g, in, out, tb);
+  constexpr int VW = sizeof(T) == 4 ? 2 : 1;
+  const unsigned grid = (unsigned)std::min<int64_t>(g.ntiles, 0x7fffffff);
+  smem = (smem + 127) & ~size_t(127);  // slots are permuted within 128 bytes
+  if (VW == 2 && g.W == 1) {
+    k_fft_mix<T, 1, true><<<grid, mix_threads(g, 1), smem, s>>>(g, in, out, tb);
+    return cudaGetLastError();
+  }
+  const int nc = g.W / VW;
+  const int nt = mix_threads(g, nc);
+  if (g.in_row || g.out_row || nc < 8)
+    k_fft_mix<T, VW, true><<<grid, nt, smem, s>>>(g, in, out, tb);
+  else
+    k_fft_mix<T, VW, false><<<grid, nt, smem, s>>>(g, in, out, tb);
   return cudaGetLastError();
 }
 

@@ -60,8 +60,7 @@ int fail(int code, const char* fmt, ...) {
 
 // digit-reversal tables of the radix plan of L (same mapping as the
 // planner's host-side tables)
-__global__ void k_gen_digits(uint16_t* p2k, uint16_t* k2p, int L) {
-  const RadixPlan rp = radix_plan(L);
+__global__ void k_gen_digits(uint16_t* p2k, uint16_t* k2p, int L, const RadixPlan rp) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < L; p += gridDim.x * blockDim.x) {
     int rem = p, k = 0, pre = 1, span = L;
     for (int s = 0; s < rp.n; ++s) {
@@ -121,6 +120,7 @@ PassGeom row_geom(int M, double scale) {
   g.ntiles = 1;
   g.tw_mode = TW_NONE;
   g.scale = scale;
+  geom_derive(g);
   return g;
 }
 
@@ -145,7 +145,7 @@ int run(const void* in, void* out, int64_t n, int direction, double scale, cudaS
   cudaError_t e = K::init_device();
   if (e == cudaSuccess) e = K::gen_twiddle(twL, M, 1, M, s);
   if (e == cudaSuccess) {
-    k_gen_digits<<<(unsigned)((M + 255) / 256), 256, 0, s>>>(p2k, k2p, (int)M);
+    k_gen_digits<<<(unsigned)((M + 255) / 256), 256, 0, s>>>(p2k, k2p, (int)M, radix_plan((int)M));
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = K::gen_chirp(chirp, n, s);

@@ -25,7 +25,7 @@
 
 namespace shafft_sm100 {
 
-constexpr int kMaxStages = 16;
+constexpr int kMaxStages = 8;
 constexpr int kMaxPassLen = 4096;
 constexpr int kThreads = 256;
 
@@ -36,60 +36,20 @@ struct RadixPlan {
   int r[kMaxStages] = {};
 };
 
-// Radix sequence for a pass of length L (L must factor into 2,3,5,7,11,13).
-// Powers of two are split into as many 8/16 stages as keep the stage count
-// minimal (512 = 8*8*8, 4096 = 16*16*16); odd primes follow.
-__host__ __device__ constexpr RadixPlan radix_plan(int L) {
-  RadixPlan p{};
-  int e = 0;
-  while (L % 2 == 0) {
-    L /= 2;
-    ++e;
-  }
-  int n16 = e / 4, rem = e % 4;
-  int pw[kMaxStages] = {};
-  int np = 0;
-  if (rem == 0) {
-    for (int i = 0; i < n16; ++i) pw[np++] = 16;
-  } else if (rem == 3) {
-    for (int i = 0; i < n16; ++i) pw[np++] = 16;
-    pw[np++] = 8;
-  } else if (rem == 2) {
-    if (n16 >= 1) {
-      for (int i = 0; i < n16 - 1; ++i) pw[np++] = 16;
-      pw[np++] = 8;
-      pw[np++] = 8;
-    } else {
-      pw[np++] = 4;
-    }
-  } else {  // rem == 1
-    if (n16 >= 2) {
-      for (int i = 0; i < n16 - 2; ++i) pw[np++] = 16;
-      pw[np++] = 8;
-      pw[np++] = 8;
-      pw[np++] = 8;
-    } else if (n16 == 1) {
-      pw[np++] = 8;
-      pw[np++] = 4;
-    } else {
-      pw[np++] = 2;
-    }
-  }
-  for (int i = 0; i < np; ++i) p.r[p.n++] = pw[i];
-  const int odd[5] = {3, 5, 7, 11, 13};
-  for (int oi = 0; oi < 5; ++oi)
-    while (L % odd[oi] == 0) {
-      L /= odd[oi];
-      p.r[p.n++] = odd[oi];
-    }
-  if (L != 1) p.n = -1;  // not representable
-  return p;
-}
+// Radix sequence of a pass of length L: radices 2 .. 13, the fewest stages
+// (each costs a trip through shared memory), among those the smallest
+// largest radix (registers), then the smallest sum; largest first.  n = 0
+// for L = 1, -1 when L has a prime factor above 13.
+RadixPlan radix_plan(int L);
 
 struct PassGeom {
   int L;
   int nst;
   int rad[kMaxStages];
+  int span[kMaxStages];       // points a block of stage s spans: L / (rad[0] .. rad[s-1])
+  uint32_t mdiv[kMaxStages];  // ceil(2^32 / d): q / d = umulhi(q, mdiv) for q, d < 2^16, with d the
+                              // butterflies of a block of stage s (the last stage: of a column)
+  int vec_in, vec_out;        // complex64: two neighbouring columns are one aligned 16-byte vector
   int W;       // tile width along b0 (power of two)
   int logW;
   int pitch;   // shared-memory row pitch in elements: element (p, w) at p*pitch + w
@@ -101,6 +61,10 @@ struct PassGeom {
   int64_t sn_in, sk_out;
   int64_t tiles_w;  // ceil(ext[0] / W)
   int64_t ntiles;   // tiles_w * ext[1] * ext[2] * ext[3]
+  // division of a tile index < 2^31 by d = tiles_w, ext[1], ext[2]:
+  // (umulhi(x, mul) + x) >> sh (tile_idx)
+  uint32_t tdiv_mul[3];
+  uint32_t tdiv_sh[3];
   int tw_mode;
   int tw_dim;
   int tw_shift;     // two-level table split: m = (m >> shift, m & mask)
@@ -129,6 +93,41 @@ struct PassGeom {
   int map_log_n, map_log_inner, map_log_q;
   int64_t map_outer;
 };
+
+// Indices of a tile: tile = tw + tiles_w * (i1 + ext[1] * (i2 + ext[2] * i3)).
+struct TileIdx {
+  int64_t tw, i1, i2, i3;
+};
+
+// Fields that follow from the others (radices, tile width, extents and
+// strides): stage spans, reciprocals, vector flags.  Call once they are set.
+void geom_derive(PassGeom& g);
+
+#ifdef __CUDACC__
+// Run-time 64-bit divisions cost a few hundred instructions a thread ahead of
+// the tile's first load; tile indices below 2^31 take multiplies instead.
+__device__ __forceinline__ TileIdx tile_idx(const PassGeom& g, int64_t tile) {
+  TileIdx x;
+  if (g.ntiles < ((int64_t)1 << 31)) {
+    const uint32_t t = (uint32_t)tile;
+    const uint32_t q0 = (__umulhi(t, g.tdiv_mul[0]) + t) >> g.tdiv_sh[0];
+    const uint32_t q1 = (__umulhi(q0, g.tdiv_mul[1]) + q0) >> g.tdiv_sh[1];
+    const uint32_t q2 = (__umulhi(q1, g.tdiv_mul[2]) + q1) >> g.tdiv_sh[2];
+    x.tw = t - q0 * (uint32_t)g.tiles_w;
+    x.i1 = q0 - q1 * (uint32_t)g.ext[1];
+    x.i2 = q1 - q2 * (uint32_t)g.ext[2];
+    x.i3 = q2;
+  } else {
+    x.tw = tile % g.tiles_w;
+    int64_t rest = tile / g.tiles_w;
+    x.i1 = rest % g.ext[1];
+    rest /= g.ext[1];
+    x.i2 = rest % g.ext[2];
+    x.i3 = rest / g.ext[2];
+  }
+  return x;
+}
+#endif
 
 enum BsMode : int { BS_LOAD_MOD = 1, BS_STORE_MULH = 2, BS_STORE_DEMOD = 4 };
 enum MapMode : int { MAP_LOAD = 1, MAP_STORE = 2 };

@@ -317,7 +317,7 @@ struct Planner {
   // radix stages of a pass of length L; nst = 0 (direct DFT) when L has a
   // prime factor above 13
   void fill_radix(PassGeom& g, int L) {
-    RadixPlan rp = radix_plan(L);
+    const RadixPlan rp = radix_plan(L);
     g.L = L;
     g.nst = rp.n > 0 ? rp.n : 0;
     for (int s = 0; s < g.nst; ++s) g.rad[s] = rp.r[s];
@@ -336,6 +336,7 @@ struct Planner {
     g.out_row = (g.sk_out == 1) ? 1 : 0;
     g.pitch = generic_pitch(W, g.in_row != 0);
     g.scale = 1.0;
+    geom_derive(g);
     st.smem = (size_t)g.L * (size_t)g.pitch * elem;
     st.tabL = ltab(g.L);
   }
@@ -1006,6 +1007,63 @@ struct Planner {
     return 0;
   }
 };
+
+// Depth-first over non-increasing radices (`best.n` < 0: none yet).
+static void radix_search(int rem, int hi, int sum, RadixPlan& cur, RadixPlan& best, int& best_sum) {
+  if (rem == 1) {
+    if (best.n < 0 || cur.n < best.n || cur.r[0] < best.r[0] || (cur.r[0] == best.r[0] && sum < best_sum)) {
+      best = cur;
+      best_sum = sum;
+    }
+    return;
+  }
+  // the rest needs at least one stage more, and as many as `hi` allows
+  int least = 0;
+  for (int p = 1; p < rem; p *= hi) ++least;
+  if (cur.n + least > (best.n > 0 ? best.n : kMaxStages)) return;
+  for (int r = hi; r >= 2; --r) {
+    if (rem % r) continue;
+    cur.r[cur.n++] = r;
+    radix_search(rem / r, r, sum + r, cur, best, best_sum);
+    cur.r[--cur.n] = 0;
+  }
+}
+
+RadixPlan radix_plan(int L) {
+  RadixPlan best, cur;
+  if (L <= 1) return best;
+  best.n = -1;
+  int best_sum = 0;
+  radix_search(L, 13, 0, cur, best, best_sum);
+  return best;
+}
+
+void geom_derive(PassGeom& g) {
+  int span = g.L;
+  for (int s = 0; s < g.nst; ++s) {
+    g.span[s] = span;
+    const bool last = s + 1 == g.nst;
+    const uint32_t d = (uint32_t)((last ? g.L : span) / g.rad[s]);
+    g.mdiv[s] = d > 1 ? (uint32_t)((((uint64_t)1 << 32) + d - 1) / d) : 0;
+    span /= g.rad[s];
+  }
+  const int64_t dv[3] = {g.tiles_w, g.ext[1], g.ext[2]};
+  for (int i = 0; i < 3; ++i) {
+    const uint64_t d = (uint64_t)std::max<int64_t>(1, std::min<int64_t>(dv[i], (int64_t)1 << 31));
+    uint32_t l = 0;
+    while (((uint64_t)1 << l) < d) ++l;
+    g.tdiv_sh[i] = l;
+    g.tdiv_mul[i] = (uint32_t)((((uint64_t)1 << 32) * (((uint64_t)1 << l) - d)) / d + 1);
+  }
+  auto vec = [&](const int64_t* st, int64_t sn) {
+    if (st[0] != 1 || sn % 2) return 0;
+    for (int d = 1; d < 4; ++d)
+      if (g.ext[d] > 1 && st[d] % 2) return 0;
+    return 1;
+  };
+  g.vec_in = vec(g.sin, g.sn_in);
+  g.vec_out = vec(g.sout, g.sk_out);
+}
 
 static void digit_tables(int L, std::vector<uint16_t>& p2k, std::vector<uint16_t>& k2p) {
   RadixPlan rp = radix_plan(L);
