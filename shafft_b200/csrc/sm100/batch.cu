@@ -345,7 +345,7 @@ int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, int 
     g.in_row = row ? 1 : 0;
     g.out_row = row ? 1 : 0;
     g.scale = 1.0;
-    geom_derive(g);
+    geom_derive(g, es);
     const size_t smem = (size_t)L * g.pitch * es;
     float ms = 0;
     for (int rep = 0; rep < 4; ++rep) {
@@ -472,7 +472,7 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
       g.in_row = row ? 1 : 0;
       g.out_row = row ? 1 : 0;
       g.scale = 1.0;
-      geom_derive(g);
+      geom_derive(g, es);
       maxsmem = std::max(maxsmem, (size_t)L * g.pitch * es);
       if (!lens.count(L)) lens[L] = LenTab{alloc(es * L), alloc(2 * L), alloc(2 * L)};
       hs.L = L;
@@ -498,7 +498,7 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
       g.ntiles = n;
       g.in_row = g.out_row = 1;
       g.scale = 1.0;
-      geom_derive(g);
+      geom_derive(g, es);
       if (!lens.count(1)) lens[1] = LenTab{alloc(es), alloc(2), alloc(2)};
       hs.L = 1;
       hs.transform = t;

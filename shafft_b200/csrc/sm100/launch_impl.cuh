@@ -480,27 +480,6 @@ SHAFFT_DEFINE_PRECISION(double, SHAFFT_FAST_LIST_F64, SHAFFT_PLANE_LIST_F64)
 #undef TYPE_
 #endif
 
-// Threads of a generic pass: the block size up to 256 that leaves the fewest
-// thread slots idle over the stages (ties to the larger block).
-static int mix_threads(const PassGeom& g, int nc) {
-  int best = 32;
-  double least = 1e30;
-  for (int nt = 32; nt <= kThreads; nt += 32) {
-    double slots = 0;
-    for (int s = 0; s < g.nst; ++s) {
-      const int nbf = g.L / g.rad[s] * nc;
-      const int rounds = (nbf + nt - 1) / nt;
-      // a block of few threads takes more rounds, each with its own latency
-      slots += (double)rounds * nt / nbf + 0.02 * rounds;
-    }
-    if (slots <= least) {
-      least = slots;
-      best = nt;
-    }
-  }
-  return best;
-}
-
 template <typename T>
 cudaError_t Launch<T>::init() {
   constexpr int kMaxSmem = 200 * 1024;
@@ -544,15 +523,18 @@ cudaError_t Launch<T>::pass(const PassGeom& g, const C* in, C* out, const PassTa
   const unsigned grid = (unsigned)std::min<int64_t>(g.ntiles, 0x7fffffff);
   smem = (smem + 127) & ~size_t(127);  // slots are permuted within 128 bytes
   if (VW == 2 && g.W == 1) {
-    k_fft_mix<T, 1, true><<<grid, mix_threads(g, 1), smem, s>>>(g, in, out, tb);
+    k_fft_mix<T, 1, true><<<grid, g.threads, smem, s>>>(g, in, out, tb);
     return cudaGetLastError();
   }
+  // The unpermuted tile spares a few instructions an access where column tiles
+  // allow it; below two waves of tiles one kernel for every pass is better
+  // (its code stays in the instruction caches from pass to pass: 8575 points
+  // complex64 9.1 us, 12.5 us with the two kernels in turn).
   const int nc = g.W / VW;
-  const int nt = mix_threads(g, nc);
-  if (g.in_row || g.out_row || nc < 8)
-    k_fft_mix<T, VW, true><<<grid, nt, smem, s>>>(g, in, out, tb);
+  if (g.in_row || g.out_row || nc < 8 || g.ntiles < 2 * 3 * 148)
+    k_fft_mix<T, VW, true><<<grid, g.threads, smem, s>>>(g, in, out, tb);
   else
-    k_fft_mix<T, VW, false><<<grid, nt, smem, s>>>(g, in, out, tb);
+    k_fft_mix<T, VW, false><<<grid, g.threads, smem, s>>>(g, in, out, tb);
   return cudaGetLastError();
 }
 

@@ -49,6 +49,7 @@ struct PassGeom {
   int span[kMaxStages];       // points a block of stage s spans: L / (rad[0] .. rad[s-1])
   uint32_t mdiv[kMaxStages];  // ceil(2^32 / d): q / d = umulhi(q, mdiv) for q, d < 2^16, with d the
                               // butterflies of a block of stage s (the last stage: of a column)
+  int threads;                // block size of the generic pass (mix_shape)
   int vec_in, vec_out;        // complex64: two neighbouring columns are one aligned 16-byte vector
   int W;       // tile width along b0 (power of two)
   int logW;
@@ -100,8 +101,17 @@ struct TileIdx {
 };
 
 // Fields that follow from the others (radices, tile width, extents and
-// strides): stage spans, reciprocals, vector flags.  Call once they are set.
-void geom_derive(PassGeom& g);
+// strides) and the element size: stage spans, reciprocals, block size, vector
+// flags.  Call once they are set.
+void geom_derive(PassGeom& g, size_t elem);
+
+// Block size of a generic pass (k_fft_mix), and its estimated time in units
+// of a point a thread.
+struct MixShape {
+  int threads;
+  double time;
+};
+MixShape mix_shape(const PassGeom& g, size_t elem);
 
 #ifdef __CUDACC__
 // Run-time 64-bit divisions cost a few hundred instructions a thread ahead of

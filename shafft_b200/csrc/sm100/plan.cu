@@ -31,6 +31,7 @@
 #include <sys/stat.h>
 
 #include <algorithm>
+#include <cmath>
 #include <atomic>
 #include <functional>
 #include <map>
@@ -199,7 +200,7 @@ struct Planner {
   // times them per shape; the defaults are the measured-best rules):
   //   balanced  multi-pass splits as balanced as possible (default for
   //             complex64) instead of the largest last factor
-  //   widen     narrower generic tiles for passes with few tiles
+  //   widen     generic tile widths by estimated time (fit_width)
   int balanced = -1;  // -1: by precision
   int widen = 1;
   // tensor-core planning: every pass of length <= 64 is a tcgen05 pass
@@ -256,16 +257,46 @@ struct Planner {
     st.smem = (size_t)g.L * 128;
   }
 
-  // Generic passes of small transforms can have too few tiles to fill the
-  // GPU: halve the tile width (down to 2) while a pass has fewer tiles than
-  // one wave of two CTAs per SM.  Measured on B200 (fwd+bwd): 121,500
-  // 0.079 -> 0.035 ms, 3^11 0.083 -> 0.045 ms, 97x64 0.062 -> 0.030 ms;
-  // passes that already have a few hundred tiles lose from narrower tiles
-  // (105^3, 1,488,375), so they are left alone.
-  void widen_grid(Step& st) {
+  // Tile width of a generic pass, given the widest one the pass would take.
+  // Radix passes: the width of the least estimated time, that of mix_shape
+  // plus the bytes an SM moves, dearer where rows are shorter than a line
+  // (column tiles on B200: 384^3 complex64 rows of 128 / 64 bytes 188 / 264
+  // us, 1536^2 complex128 64 / 32 bytes 31 / 39 us).
+  // Tiles up to 96 KiB (two CTAs an SM) where rows would be under 64 bytes.
+  // Direct-DFT passes: halve the width (down to 2) while there are fewer
+  // tiles than one wave of two CTAs per SM (97x64 complex64 0.062 -> 0.030 ms
+  // fwd+bwd; passes with a few hundred tiles lose from narrower ones).
+  void fit_width(Step& st) {
     if (!widen || st.fast || st.tc || st.kind != ST_PASS) return;
-    const int64_t want = 2 * 148;
-    while (st.g.W > 2 && st.g.ntiles < want) finish_geom(st, st.g.W / 2);
+    PassGeom& g = st.g;
+    if (g.nst == 0) {
+      while (g.W > 2 && g.ntiles < 2 * 148) finish_geom(st, g.W / 2);
+      return;
+    }
+    const int wide = g.W, narrow = std::min(wide, vw());
+    int best = wide;
+    double least = -1;
+    const bool rows_in = g.in_row != 0, rows_out = g.out_row != 0;
+    // candidates: the width given, narrower ones, last the double width
+    std::vector<int> cand;
+    for (int w = wide; w >= narrow && w > 0; w /= 2) cand.push_back(w);
+    if (wide * (int)elem < 64 && wide * 2 <= pow2ceil(g.ext[0]) && (size_t)g.L * wide * 2 * elem <= (96 << 10) &&
+        !rows_in && !rows_out)
+      cand.push_back(wide * 2);
+    for (const int w : cand) {
+      finish_geom(st, w);
+      const MixShape sh = mix_shape(g, elem);
+      double t = sh.time;
+      const double row = (double)w * elem;
+      const double dear = row >= 128 ? 1.0 : row >= 64 ? 1.3 : row >= 32 ? 2.0 : 3.2;
+      const double sm_bytes = std::ceil(g.ntiles / 148.0) * g.L * w * elem;
+      t += sm_bytes * 1.2e-4 * 0.5 * ((rows_in ? 1.0 : dear) + (rows_out ? 1.0 : dear));
+      if (least < 0 || t < least * 0.92) {
+        least = t;
+        best = w;
+      }
+    }
+    finish_geom(st, best);
   }
 
   void mark_tc(Step& st) {
@@ -336,7 +367,7 @@ struct Planner {
     g.out_row = (g.sk_out == 1) ? 1 : 0;
     g.pitch = generic_pitch(W, g.in_row != 0);
     g.scale = 1.0;
-    geom_derive(g);
+    geom_derive(g, elem);
     st.smem = (size_t)g.L * (size_t)g.pitch * elem;
     st.tabL = ltab(g.L);
   }
@@ -367,7 +398,7 @@ struct Planner {
       g.sn_in = g.sk_out = 1;
       finish_geom(st, W);
       if (cur_tc) mark_tc(st);
-      widen_grid(st);
+      fit_width(st);
     } else {
       int W = col_width(L, I);
       g.ext[0] = I;
@@ -378,7 +409,7 @@ struct Planner {
       g.sn_in = g.sk_out = I;
       finish_geom(st, W);
       try_fast(st);
-      widen_grid(st);
+      fit_width(st);
     }
     out.push_back(st);
   }
@@ -580,7 +611,7 @@ struct Planner {
       st.tabN = ntab(span);
       finish_geom(st, W);
       try_fast(st);
-      widen_grid(st);
+      fit_width(st);
       out.push_back(st);
       span = m;
     }
@@ -628,7 +659,7 @@ struct Planner {
       }
       finish_geom(st, W);
       try_fast(st);
-      widen_grid(st);
+      fit_width(st);
       out.push_back(st);
     }
   }
@@ -1038,7 +1069,39 @@ RadixPlan radix_plan(int L) {
   return best;
 }
 
-void geom_derive(PassGeom& g) {
+// Block sizes of 32 .. 256 threads are compared by an estimate of the pass's
+// time: waves of resident tiles (shared memory; 768 threads an SM at 80
+// registers), a part wave counting as at least half of one, times the points
+// a busy thread handles in a tile plus the tile's own latency (first loads
+// and barriers, about six points' worth).  Measured on B200, 384^3 complex64
+// column passes (48 KiB tiles, four CTAs): 192 threads 184 us, 128 (no idle
+// slot, but 512 threads resident) 207, 256 (a quarter idle) 207; 1225 x 1215
+// complex128 rows: 128 threads (one wave) 22.7 us, 192 (1.03 waves) 23.9.
+MixShape mix_shape(const PassGeom& g, size_t elem) {
+  const int nc = elem == 16 || g.W == 1 ? g.W : g.W / 2;
+  const size_t smem = (size_t)g.L * g.pitch * elem;
+  const int fit = std::max(1, std::min(32, (int)((227 << 10) / (smem + 1024))));
+  MixShape best{32, -1};
+  for (int nt = kThreads; nt >= 32; nt -= 32) {
+    const int ctas = std::max(1, std::min(fit, 768 / nt));
+    double slots = 0, work = 0;
+    for (int s = 0; s < g.nst; ++s) {
+      const int nbf = g.L / g.rad[s] * nc;
+      slots += (double)((nbf + nt - 1) / nt * nt);
+      work += nbf;
+    }
+    const double busy = slots > 0 ? nt * work / slots : nt;
+    const double waves = (double)g.ntiles / (148.0 * ctas);
+    const double rest = std::ceil((waves - std::floor(waves)) * ctas - 1e-9) / ctas;
+    const double t =
+        (std::floor(waves) + (rest > 0 ? std::max(0.5, rest) : 0.0)) * ((double)g.L * g.W / busy + 6.0);
+    if (best.time < 0 || t < best.time * 0.999) best = MixShape{nt, t};
+  }
+  return best;
+}
+
+void geom_derive(PassGeom& g, size_t elem) {
+  g.threads = g.nst > 0 ? mix_shape(g, elem).threads : kThreads;
   int span = g.L;
   for (int s = 0; s < g.nst; ++s) {
     g.span[s] = span;
