@@ -346,11 +346,10 @@ int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, int 
     g.out_row = row ? 1 : 0;
     g.scale = 1.0;
     geom_derive(g, es);
-    const size_t smem = (size_t)L * g.pitch * es;
     float ms = 0;
     for (int rep = 0; rep < 4; ++rep) {
       cudaEventRecord(e0);
-      Launch<T>::pass(g, a, b, tb, smem, nullptr);
+      Launch<T>::pass(g, a, b, tb, nullptr);
       cudaEventRecord(e1);
       cudaEventSynchronize(e1);
       float t = 0;
@@ -473,7 +472,7 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
       g.out_row = row ? 1 : 0;
       g.scale = 1.0;
       geom_derive(g, es);
-      maxsmem = std::max(maxsmem, (size_t)L * g.pitch * es);
+      maxsmem = std::max(maxsmem, pass_smem(g, es));
       if (!lens.count(L)) lens[L] = LenTab{alloc(es * L), alloc(2 * L), alloc(2 * L)};
       hs.L = L;
       hs.transform = t;
@@ -596,7 +595,7 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
     BCUDA(cudaMalloc(&b->d_tslot, sizeof(int) * std::max<size_t>(ts.size(), 1)));
     if (!ts.empty()) BCUDA(cudaMemcpy(b->d_tslot, ts.data(), sizeof(int) * ts.size(), cudaMemcpyHostToDevice));
   }
-  b->smem = std::max<size_t>((maxsmem + 127) & ~size_t(127), 128);  // slots are permuted within 128 bytes
+  b->smem = std::max<size_t>(maxsmem, 128);
   BCUDA(cudaFuncSetAttribute(k_fft_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)std::max<size_t>(b->smem, 48 * 1024)));
   int dev = 0, sms = 148, per = 1;

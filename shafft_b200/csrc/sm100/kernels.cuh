@@ -14,123 +14,190 @@
 
 namespace shafft_sm100 {
 
+// Cosine c and sine s of a direct DFT, and acc + a * c, acc + a * s on complex
+// numbers: for complex64 one packed FMA for both parts (two roundings as of
+// two scalar FMAs), whose operand is the factor twice.
+template <typename C>
+struct DirectTw;
+template <>
+struct alignas(16) DirectTw<float2> {
+  float2 cc, ss;
+  __device__ __forceinline__ void set(float2 t) {
+    cc = float2{t.x, t.x};
+    ss = float2{t.y, t.y};
+  }
+  static __device__ __forceinline__ float2 fma2(float2 a, float2 tt, float2 acc) {
+    float2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<unsigned long long&>(r))
+        : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(tt)),
+          "l"(reinterpret_cast<const unsigned long long&>(acc)));
+    return r;
+  }
+  __device__ __forceinline__ float2 add_c(float2 a, float2 acc) const { return fma2(a, cc, acc); }
+  __device__ __forceinline__ float2 add_s(float2 a, float2 acc) const { return fma2(a, ss, acc); }
+};
+template <>
+struct alignas(16) DirectTw<double2> {
+  double2 t;
+  __device__ __forceinline__ void set(double2 x) { t = x; }
+  __device__ __forceinline__ double2 add_c(double2 a, double2 acc) const {
+    return double2{fma(a.x, t.x, acc.x), fma(a.y, t.x, acc.y)};
+  }
+  __device__ __forceinline__ double2 add_s(double2 a, double2 acc) const {
+    return double2{fma(a.x, t.y, acc.x), fma(a.y, t.y, acc.y)};
+  }
+};
+
 // One output of a direct-DFT tile, with the pass's fused post-twiddle,
 // scale and output conjugation.
 template <typename T, typename C>
 __device__ __forceinline__ void direct_put(const PassGeom& g, const PassTables<C>& tb, C* out, C y, int k, int w,
-                                           int64_t bout, int64_t w0, int64_t tconst, T scale) {
+                                           const TileAt& at, T scale) {
   if (g.tw_mode == TW_POST) {
-    const int64_t tt = (g.tw_dim == 0) ? (w0 + w) : tconst;
+    const int64_t tt = (g.tw_dim == 0) ? (at.w0 + w) : at.tconst;
     y = cmul(y, tw_n(tb, g.tw_shift, g.tw_mask, (int64_t)k * tt));
   }
-  if (g.scale != 1.0) y = cscale(y, scale);
-  if (g.conj_out) y.y = -y.y;
-  out[bout + (int64_t)w * g.sout[0] + (int64_t)k * g.sk_out] = y;
+  y = C{y.x * scale, g.conj_out ? -(y.y * scale) : y.y * scale};
+  out[at.bout + (int64_t)w * g.sout[0] + (int64_t)k * g.sk_out] = y;
 }
 
-// Direct DFT of the tile held in shared memory (natural order, [n][w] with
-// the given pitch), X[k] = sum_n x[n] w^{nk} with w = exp(-2 pi i / L),
-// evaluated in pairs.  With s[n] = x[n] + x[L-n] and d[n] = x[n] - x[L-n]
-// for n = 1 .. h (h = (L-1)/2), and e_k = (-1)^k x[L/2] for even L (0 for
-// odd L):
+// Sums and stores of a direct-DFT tile: item (jg, wg) is the output pairs
+// jg + i * ng (i < J) of the columns wg + c * WG (c < CB).
+template <typename T, int J, int CB>
+__device__ __forceinline__ void direct_sums(const PassGeom& g, const PassTables<typename Cx<T>::type>& tb,
+                                            typename Cx<T>::type* out, const typename Cx<T>::type* sm,
+                                            const DirectTw<typename Cx<T>::type>* tw, const TileAt& at) {
+  using C = typename Cx<T>::type;
+  const int L = g.L, W = g.W, pitch = g.pitch;
+  const int h = (L - 1) / 2, half = L / 2, np = half + 1;
+  const bool even = (L & 1) == 0;
+  const T scale = (T)g.scale;
+  const int WG = W >= CB ? W / CB : 1, ng = (np + J - 1) / J;
+  const int logWG = W >= CB ? g.logW - (CB == 2 ? 1 : 0) : 0;
+  for (int b = threadIdx.x; b < (ng << logWG); b += blockDim.x) {
+    const int wg = b & (WG - 1), jg = b >> logWG;
+    if (wg >= at.wcount) continue;
+    C P[J][CB], Q[J][CB];
+    int j[J], m[J];
+#pragma unroll
+    for (int i = 0; i < J; ++i) {
+      j[i] = min(jg + i * ng, half);
+      m[i] = 0;
+#pragma unroll
+      for (int c = 0; c < CB; ++c) P[i][c] = Q[i][c] = C{0, 0};
+    }
+    auto step = [&](int n) {
+      C sn[CB], dn[CB];
+#pragma unroll
+      for (int c = 0; c < CB; ++c) {
+        const int w = min(wg + c * WG, W - 1);
+        sn[c] = sm[n * pitch + w];
+        dn[c] = sm[(L - n) * pitch + w];
+      }
+#pragma unroll
+      for (int i = 0; i < J; ++i) {
+        const uint32_t mi = (uint32_t)(m[i] + j[i]);
+        m[i] = (int)min(mi, mi - (uint32_t)L);  // mod L: mi - L wraps to a large number below L
+        const DirectTw<C> t = tw[m[i]];
+#pragma unroll
+        for (int c = 0; c < CB; ++c) {
+          P[i][c] = t.add_c(sn[c], P[i][c]);
+          Q[i][c] = t.add_s(dn[c], Q[i][c]);
+        }
+      }
+    };
+    if constexpr (J == 1) {
+#pragma unroll 4  // a lone output pair waits on its own loads
+      for (int n = 1; n <= h; ++n) step(n);
+    } else {
+      for (int n = 1; n <= h; ++n) step(n);
+    }
+#pragma unroll
+    for (int c = 0; c < CB; ++c) {
+      const int w = wg + c * WG;
+      if (w >= at.wcount) continue;
+      const C x0 = sm[w];
+      const C xh = even ? sm[half * pitch + w] : C{0, 0};
+#pragma unroll
+      for (int i = 0; i < J; ++i) {
+        const int k = jg + i * ng;
+        if (k > half) continue;
+        const T e = (k & 1) ? (T)-1 : (T)1;
+        const T bx = x0.x + e * xh.x + P[i][c].x, by = x0.y + e * xh.y + P[i][c].y;
+        direct_put<T, C>(g, tb, out, C{bx - Q[i][c].y, by + Q[i][c].x}, k, w, at, scale);
+        if (k > 0 && 2 * k != L)
+          direct_put<T, C>(g, tb, out, C{bx + Q[i][c].y, by - Q[i][c].x}, L - k, w, at, scale);
+      }
+    }
+  }
+}
+
+// One tile of a direct-DFT pass: X[k] = sum_n x[n] w^{nk}, w = exp(-2 pi i / L),
+// evaluated in pairs.  With s[n] = x[n] + x[L-n] and d[n] = x[n] - x[L-n] for
+// n = 1 .. h (h = (L-1)/2), and e_k = (-1)^k x[L/2] for even L (0 for odd L):
 //   X[k]   = x[0] + e_k + sum_n s[n] Re w^{nk} + i sum_n d[n] Im w^{nk}
 //   X[L-k] = x[0] + e_k + sum_n s[n] Re w^{nk} - i sum_n d[n] Im w^{nk}
-// for k = 1 .. h; X[0] = x[0] + sum_n s[n] + x[L/2] and, for even L,
-// X[L/2] = x[0] + sum_n (-1)^n s[n] + (-1)^{L/2} x[L/2].  Each table read
-// and each pair of real multiplies then serves two outputs, a quarter of
-// the arithmetic of the plain sum; the exponent n*k is reduced modulo L
-// incrementally.  Used for lengths with a prime factor above 13 when L is
-// small enough that O(L) work per output beats a Bluestein round trip.
-// Outputs go straight to HBM with the pass's fused twiddle/scale/conj.
-template <typename T, typename C>
-__device__ __forceinline__ void direct_store(const PassGeom& g, const PassTables<C>& tb, C* sm, C* out, int L,
-                                             int W, int logW, int pitch, int wcount, int64_t bout, int64_t w0,
-                                             int64_t tconst) {
-  const int h = (L - 1) / 2;
-  const bool even = (L & 1) == 0;
-  // s and d in place: row n <- s[n], row L-n <- d[n]
-  for (int b = threadIdx.x; b < (h << logW); b += kThreads) {
-    const int w = b & (W - 1), n = 1 + (b >> logW);
-    const C a = sm[n * pitch + w], c = sm[(L - n) * pitch + w];
-    sm[n * pitch + w] = C{a.x + c.x, a.y + c.y};
-    sm[(L - n) * pitch + w] = C{a.x - c.x, a.y - c.y};
-  }
-  __syncthreads();
-  const T scale = (T)g.scale;
-  // item (j, w): j = 0 gives X[0] (and X[L/2] for even L), j = 1 .. h gives
-  // X[j] and X[L-j]
-  const int items = (h + 1) << logW;
-  for (int b = threadIdx.x; b < items; b += kThreads) {
-    const int w = b & (W - 1), j = b >> logW;
-    if (w >= wcount) continue;
-    const C x0 = sm[w];
-    const C xh = even ? sm[(L / 2) * pitch + w] : C{0, 0};
-    if (j == 0) {
-      C y0 = x0, yh = x0;
-      T sg = -1;
-      for (int n = 1; n <= h; ++n) {
-        const C sn = sm[n * pitch + w];
-        y0.x += sn.x;
-        y0.y += sn.y;
-        yh.x += sg * sn.x;
-        yh.y += sg * sn.y;
-        sg = -sg;
-      }
-      y0.x += xh.x;
-      y0.y += xh.y;
-      direct_put<T, C>(g, tb, out, y0, 0, w, bout, w0, tconst, scale);
-      if (even) {
-        const T e = ((L / 2) & 1) ? (T)-1 : (T)1;
-        yh.x += e * xh.x;
-        yh.y += e * xh.y;
-        direct_put<T, C>(g, tb, out, yh, L / 2, w, bout, w0, tconst, scale);
-      }
-      continue;
-    }
-    T px = 0, py = 0, qx = 0, qy = 0;
-    int m = 0;
-    for (int n = 1; n <= h; ++n) {
-      m += j;
-      if (m >= L) m -= L;
-      const C t = tb.twL[m];
-      const C sn = sm[n * pitch + w], dn = sm[(L - n) * pitch + w];
-      px += sn.x * t.x;
-      py += sn.y * t.x;
-      qx += dn.x * t.y;
-      qy += dn.y * t.y;
-    }
-    const T e = (j & 1) ? (T)-1 : (T)1;
-    const T bx = x0.x + e * xh.x + px, by = x0.y + e * xh.y + py;
-    direct_put<T, C>(g, tb, out, C{bx - qy, by + qx}, j, w, bout, w0, tconst, scale);
-    direct_put<T, C>(g, tb, out, C{bx + qy, by - qx}, L - j, w, bout, w0, tconst, scale);
-  }
-}
-
-// One tile of a direct-DFT pass.  `sm` holds L * pitch elements.
+// for k = 0 .. L/2 (X[0], and X[L/2] of even L, are their own partners): two
+// real h x h matrices times the complex columns s and d, a quarter of the
+// arithmetic of the plain sum.  Used for lengths with a prime factor above 13
+// when L is small enough that O(L) work per output beats a Bluestein round
+// trip.
+//
+// Bound by FP32 / FP64 multiply-adds (about L per point), so a thread keeps
+// kDirectJ output pairs of direct_cols columns in registers: each twiddle pair read
+// serves the columns and each s, d the outputs, and complex64 sums take one
+// packed multiply-add for both parts.  The exponent n*k is reduced modulo L
+// incrementally.
+//
+// `sm` holds the tile, L * pitch elements ([n][w]; rows n and L - n hold s and
+// d), rounded up to 16 bytes, then L DirectTw.
 template <typename T>
 __device__ __forceinline__ void direct_tile(const PassGeom& g, const typename Cx<T>::type* in,
                                             typename Cx<T>::type* out,
                                             const PassTables<typename Cx<T>::type>& tb, int64_t tile,
                                             typename Cx<T>::type* sm) {
   using C = typename Cx<T>::type;
-  const int L = g.L, W = g.W;
+  const int L = g.L, W = g.W, pitch = g.pitch;
+  const int half = L / 2;
   const TileAt at = tile_at(g, tile);
-  const int total = L << g.logW;
-  for (int b = threadIdx.x; b < total; b += kThreads) {
+  DirectTw<C>* tw = reinterpret_cast<DirectTw<C>*>(
+      reinterpret_cast<unsigned char*>(sm) + (((size_t)L * pitch * sizeof(C) + 15) & ~(size_t)15));
+  for (int m = threadIdx.x; m < L; m += blockDim.x) tw[m].set(__ldg(tb.twL + m));
+  // s and d of the pairs (n, L - n); n = 0 and, for even L, L/2 alone
+  const int np = half + 1;
+  const T sy = g.conj_in ? (T)-1 : (T)1;
+#pragma unroll 2
+  for (int b = threadIdx.x; b < (np << g.logW); b += blockDim.x) {
     int w, n;
     if (g.in_row) {
-      n = b % L;
-      w = b / L;
+      w = np > 1 ? (int)__umulhi((uint32_t)b, g.mdiv[0]) : b;
+      n = b - w * np;
     } else {
       w = b & (W - 1);
       n = b >> g.logW;
     }
-    C x = (w < at.wcount) ? in[at.bin + (int64_t)w * g.sin[0] + (int64_t)n * g.sn_in] : C{0, 0};
-    if (g.conj_in) x.y = -x.y;
-    sm[n * g.pitch + w] = x;
+    const int n2 = n == 0 ? 0 : L - n;
+    const C* p = in + at.bin + (int64_t)w * g.sin[0];
+    C x = C{0, 0}, z = C{0, 0};
+    if (w < at.wcount) {
+      x = p[(int64_t)n * g.sn_in];
+      if (n != n2) z = p[(int64_t)n2 * g.sn_in];
+    }
+    x.y *= sy;
+    z.y *= sy;
+    if (n == n2) {
+      sm[n * pitch + w] = x;
+    } else {
+      sm[n * pitch + w] = C{x.x + z.x, x.y + z.y};
+      sm[n2 * pitch + w] = C{x.x - z.x, x.y - z.y};
+    }
   }
   __syncthreads();
-  direct_store<T, C>(g, tb, sm, out, L, W, g.logW, g.pitch, at.wcount, at.bout, at.w0, at.tconst);
+  if (g.direct_j == 1)
+    direct_sums<T, 1, 1>(g, tb, out, sm, tw, at);
+  else
+    direct_sums<T, kDirectJ, direct_cols(sizeof(C))>(g, tb, out, sm, tw, at);
 }
 
 template <typename T>

@@ -81,7 +81,7 @@ struct Launch {
   // them on every one (thread-safe; later calls return the first result)
   static cudaError_t init_device();
   static cudaError_t pass(const PassGeom& g, const C* in, C* out, const PassTables<C>& tb,
-                          size_t smem, cudaStream_t s);
+                          cudaStream_t s);
   // specialised pass for a hot length; tile width is 16 bytes x 8 (= 8*VW
   // elements), output is a column tile.  Returns cudaErrorNotSupported when
   // no specialisation exists for L.

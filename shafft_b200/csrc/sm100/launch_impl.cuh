@@ -513,15 +513,15 @@ cudaError_t Launch<T>::init_device() {
 
 template <typename T>
 cudaError_t Launch<T>::pass(const PassGeom& g, const C* in, C* out, const PassTables<C>& tb,
-                            size_t smem, cudaStream_t s) {
+                            cudaStream_t s) {
+  const size_t smem = pass_smem(g, sizeof(C));
   if (g.nst == 0) {
     const int64_t grid = std::min<int64_t>(g.ntiles, 148 * 64);
-    k_fft_direct<T><<<(unsigned)grid, kThreads, smem, s>>>(g, in, out, tb);
+    k_fft_direct<T><<<(unsigned)grid, g.threads, smem, s>>>(g, in, out, tb);
     return cudaGetLastError();
   }
   constexpr int VW = sizeof(T) == 4 ? 2 : 1;
   const unsigned grid = (unsigned)std::min<int64_t>(g.ntiles, 0x7fffffff);
-  smem = (smem + 127) & ~size_t(127);  // slots are permuted within 128 bytes
   if (VW == 2 && g.W == 1) {
     k_fft_mix<T, 1, true><<<grid, g.threads, smem, s>>>(g, in, out, tb);
     return cudaGetLastError();

@@ -154,15 +154,14 @@ int run(const void* in, void* out, int64_t n, int direction, double scale, cudaS
   tb.twL = twL;
   tb.p2k = p2k;
   tb.k2p = k2p;
-  const size_t smem = (size_t)M * sizeof(C);
   // H = FFT_M(h) / M
-  if (e == cudaSuccess) e = K::pass(row_geom((int)M, 1.0 / (double)M, sizeof(C)), S0, H, tb, smem, s);
+  if (e == cudaSuccess) e = K::pass(row_geom((int)M, 1.0 / (double)M, sizeof(C)), S0, H, tb, s);
   // modulate (writes all M entries: the zero padding included)
   if (e == cudaSuccess)
     e = K::bs_modulate(reinterpret_cast<const C*>(in), S0, n, M, 1, M, chirp, direction, s);
-  if (e == cudaSuccess) e = K::pass(row_geom((int)M, 1.0, sizeof(C)), S0, S1, tb, smem, s);
+  if (e == cudaSuccess) e = K::pass(row_geom((int)M, 1.0, sizeof(C)), S0, S1, tb, s);
   if (e == cudaSuccess) e = K::bs_mulh(S1, H, M, M, s);
-  if (e == cudaSuccess) e = K::pass(row_geom((int)M, 1.0, sizeof(C)), S1, S0, tb, smem, s);
+  if (e == cudaSuccess) e = K::pass(row_geom((int)M, 1.0, sizeof(C)), S1, S0, tb, s);
   if (e == cudaSuccess)
     e = K::bs_demod(S0, reinterpret_cast<C*>(out), n, M, 1, n, chirp, direction, (T)scale, s);
   if (e != cudaSuccess) return fail(SHAFFT_SM100_ECUDA, "launch: %s", cudaGetErrorString(e));

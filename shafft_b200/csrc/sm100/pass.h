@@ -42,14 +42,16 @@ struct RadixPlan {
 // for L = 1, -1 when L has a prime factor above 13.
 RadixPlan radix_plan(int L);
 
-struct PassGeom {
+struct alignas(16) PassGeom {
   int L;
   int nst;
   int rad[kMaxStages];
   int span[kMaxStages];       // points a block of stage s spans: L / (rad[0] .. rad[s-1])
   uint32_t mdiv[kMaxStages];  // ceil(2^32 / d): q / d = umulhi(q, mdiv) for q, d < 2^16, with d the
-                              // butterflies of a block of stage s (the last stage: of a column)
+                              // butterflies of a block of stage s (the last stage: of a column); direct
+                              // DFT: mdiv[0] for d = L / 2 + 1
   int threads;                // block size of the generic pass (mix_shape)
+  int direct_j;               // direct DFT: output pairs a thread works on at a time (1 or kDirectJ)
   int vec_in, vec_out;        // complex64: two neighbouring columns are one aligned 16-byte vector
   int W;       // tile width along b0 (power of two)
   int logW;
@@ -105,13 +107,24 @@ struct TileIdx {
 // flags.  Call once they are set.
 void geom_derive(PassGeom& g, size_t elem);
 
-// Block size of a generic pass (k_fft_mix), and its estimated time in units
-// of a point a thread.
+// Dynamic shared memory of a generic (k_fft_mix) or direct-DFT pass.
+size_t pass_smem(const PassGeom& g, size_t elem);
+
+// Outputs a thread of a direct-DFT tile works on at a time: kDirectJ output
+// pairs (k, L - k) of direct_cols columns, or one of one where the tiles are
+// too few to keep an SM busy that way.
+constexpr int kDirectJ = 4;
+__host__ __device__ constexpr int direct_cols(size_t elem) { return elem == 8 ? 2 : 1; }
+
+// Block size of a generic (k_fft_mix) or direct-DFT pass, and its estimated
+// time (arbitrary units, comparable between widths of one pass).
 struct MixShape {
   int threads;
   double time;
+  int direct_j = 0;
 };
 MixShape mix_shape(const PassGeom& g, size_t elem);
+MixShape direct_shape(const PassGeom& g, size_t elem);
 
 #ifdef __CUDACC__
 // Run-time 64-bit divisions cost a few hundred instructions a thread ahead of

@@ -263,35 +263,31 @@ struct Planner {
   // (column tiles on B200: 384^3 complex64 rows of 128 / 64 bytes 188 / 264
   // us, 1536^2 complex128 64 / 32 bytes 31 / 39 us).
   // Tiles up to 96 KiB (two CTAs an SM) where rows would be under 64 bytes.
-  // Direct-DFT passes: halve the width (down to 2) while there are fewer
-  // tiles than one wave of two CTAs per SM (97x64 complex64 0.062 -> 0.030 ms
-  // fwd+bwd; passes with a few hundred tiles lose from narrower ones).
+  // Direct-DFT passes likewise by direct_shape, from columns up to 64 wide
+  // (a thread holds several outputs, so short lengths need many columns).
   void fit_width(Step& st) {
     if (!widen || st.fast || st.tc || st.kind != ST_PASS) return;
     PassGeom& g = st.g;
-    if (g.nst == 0) {
-      while (g.W > 2 && g.ntiles < 2 * 148) finish_geom(st, g.W / 2);
-      return;
-    }
-    const int wide = g.W, narrow = std::min(wide, vw());
+    const bool direct = g.nst == 0;
+    const int wide = direct ? std::max(g.W, std::min({64, pow2floor(lim.e_target / g.L), pow2ceil(g.ext[0])})) : g.W;
+    const int narrow = std::min(wide, vw());
     int best = wide;
     double least = -1;
     const bool rows_in = g.in_row != 0, rows_out = g.out_row != 0;
     // candidates: the width given, narrower ones, last the double width
     std::vector<int> cand;
     for (int w = wide; w >= narrow && w > 0; w /= 2) cand.push_back(w);
-    if (wide * (int)elem < 64 && wide * 2 <= pow2ceil(g.ext[0]) && (size_t)g.L * wide * 2 * elem <= (96 << 10) &&
+    if (!direct && wide * (int)elem < 64 && wide * 2 <= pow2ceil(g.ext[0]) && (size_t)g.L * wide * 2 * elem <= (96 << 10) &&
         !rows_in && !rows_out)
       cand.push_back(wide * 2);
     for (const int w : cand) {
       finish_geom(st, w);
-      const MixShape sh = mix_shape(g, elem);
-      double t = sh.time;
+      double t = (direct ? direct_shape(g, elem) : mix_shape(g, elem)).time;
       const double row = (double)w * elem;
       const double dear = row >= 128 ? 1.0 : row >= 64 ? 1.3 : row >= 32 ? 2.0 : 3.2;
       const double sm_bytes = std::ceil(g.ntiles / 148.0) * g.L * w * elem;
-      t += sm_bytes * 1.2e-4 * 0.5 * ((rows_in ? 1.0 : dear) + (rows_out ? 1.0 : dear));
-      if (least < 0 || t < least * 0.92) {
+      t += sm_bytes * (direct ? 0.02 : 1.2e-4) * 0.5 * ((rows_in ? 1.0 : dear) + (rows_out ? 1.0 : dear));
+      if (least < 0 || t < least * (direct ? 0.85 : 0.92)) {
         least = t;
         best = w;
       }
@@ -1100,8 +1096,50 @@ MixShape mix_shape(const PassGeom& g, size_t elem) {
   return best;
 }
 
+// Waves of resident tiles times a tile's time: rounds of loads, then the sums,
+// the longer of a warp's own chain (120 / 60 cycles a step with kDirectJ / one
+// output pair a thread) and the issue slots of the warps that share a
+// scheduler (34 a step for complex64, 45 for complex128 with its half-rate
+// FP64 pipe; 12 / 14 for one).
+MixShape direct_shape(const PassGeom& g, size_t elem) {
+  MixShape best{32, -1, 1};
+  for (const int j : {kDirectJ, 1}) {
+    const int cols = j == 1 ? 1 : direct_cols(elem);
+    const int pairs = g.L / 2 + 1;
+    const int items = (pairs + j - 1) / j * std::max(1, g.W / cols);
+    // threads for the sums, or more where the loads are what takes long
+    for (const int want : {items, std::max(items, pairs * g.W / 2)}) {
+      const int nt = std::max(32, std::min(kThreads, (want + 31) / 32 * 32));
+      const int fit = (int)((227 << 10) / (pass_smem(g, elem) + 1024));
+      const int ctas = std::max(1, std::min({fit, 65536 / (nt * 80), 32}));
+      const double rounds = std::ceil((double)items / nt);
+      const double busy = std::min(items, nt) / 128.0;  // warps a scheduler has of one tile
+      const double chain = j == 1 ? 60.0 : 120.0;
+      const double issue = j == 1 ? (elem == 8 ? 12.0 : 14.0) : (elem == 8 ? 34.0 : 45.0);
+      auto wave = [&](double c) {
+        const double load = 700.0 * std::ceil((double)pairs * g.W / (2 * nt)) + 0.1 * c * g.L * g.W;
+        return load + (g.L - 1) / 2 * rounds * std::max(chain, issue * std::max(1.0, c * busy)) + 1000.0;
+      };
+      const double waves = (double)g.ntiles / (148.0 * ctas);
+      const double rest = std::ceil((waves - std::floor(waves)) * ctas - 1e-9);
+      const double t = std::floor(waves) * wave(ctas) + (rest > 0 ? wave(rest) : 0.0);
+      if (best.time < 0 || t < best.time) best = MixShape{nt, t, j};
+    }
+  }
+  return best;
+}
+
+size_t pass_smem(const PassGeom& g, size_t elem) {
+  const size_t tile = (size_t)g.L * g.pitch * elem;
+  // slots of radix passes are permuted within 128 bytes; direct-DFT passes
+  // keep their twiddles behind the tile
+  return g.nst > 0 ? (tile + 127) & ~size_t(127) : ((tile + 15) & ~size_t(15)) + 16 * (size_t)g.L;
+}
+
 void geom_derive(PassGeom& g, size_t elem) {
-  g.threads = g.nst > 0 ? mix_shape(g, elem).threads : kThreads;
+  const MixShape sh = g.nst > 0 ? mix_shape(g, elem) : direct_shape(g, elem);
+  g.threads = sh.threads;
+  g.direct_j = sh.direct_j;
   int span = g.L;
   for (int s = 0; s < g.nst; ++s) {
     g.span[s] = span;
@@ -1109,6 +1147,10 @@ void geom_derive(PassGeom& g, size_t elem) {
     const uint32_t d = (uint32_t)((last ? g.L : span) / g.rad[s]);
     g.mdiv[s] = d > 1 ? (uint32_t)((((uint64_t)1 << 32) + d - 1) / d) : 0;
     span /= g.rad[s];
+  }
+  if (g.nst == 0) {  // direct DFT: row tiles are loaded in L / 2 + 1 pairs a row
+    const uint32_t d = (uint32_t)g.L / 2 + 1;
+    g.mdiv[0] = (uint32_t)((((uint64_t)1 << 32) + d - 1) / d);
   }
   const int64_t dv[3] = {g.tiles_w, g.ext[1], g.ext[2]};
   for (int i = 0; i < 3; ++i) {
@@ -1265,8 +1307,7 @@ struct Launcher {
                            reinterpret_cast<C*>(out), tables(p, st),
                            reinterpret_cast<int*>(p->d_tables + p->off_tcerr), s),
                    "fast fft pass");
-    return check(K::pass(g, reinterpret_cast<const C*>(in), reinterpret_cast<C*>(out), tables(p, st),
-                         st.smem, s),
+    return check(K::pass(g, reinterpret_cast<const C*>(in), reinterpret_cast<C*>(out), tables(p, st), s),
                  "fft pass");
   }
 

@@ -64,3 +64,14 @@ def test_batch_buffers_on_8_bytes(offset):
             assert o.rel_l2(y.reshape(x.shape), o.fftn(x.astype(np.complex128))) <= _tol(x.size, S.C2C)
     for y0, y1 in zip(*outs):
         assert np.array_equal(y0, y1)
+
+
+# both forms of the sums (four output pairs a thread, one), even lengths with
+# their middle output, rows and columns, ragged tiles
+DIRECT = [(17, 40), (34, 17), (97, 6), (362,), (353, 3), (211, 64, 31), (46, 58, 62), (2, 19), (64, 64, 61)]
+
+
+@pytest.mark.parametrize("prec", [S.C2C, S.Z2Z])
+@pytest.mark.parametrize("dims", DIRECT, ids=lambda d: "x".join(map(str, d)))
+def test_direct_pass_matches_oracle(dims, prec):
+    test_generic_pass_matches_oracle(dims, prec)
