@@ -213,22 +213,57 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// streaming accesses of 8- and 16-byte vectors
+template <typename V>
+__device__ __forceinline__ V ld_vec(const V* p) {
+  static_assert(sizeof(V) == 16 || sizeof(V) == 8, "vector of 8 or 16 bytes");
+  V v;
+  if constexpr (sizeof(V) == 16)
+    reinterpret_cast<float4&>(v) = __ldcs(reinterpret_cast<const float4*>(p));
+  else
+    reinterpret_cast<float2&>(v) = __ldcs(reinterpret_cast<const float2*>(p));
+  return v;
+}
+template <typename V>
+__device__ __forceinline__ void st_vec(V* p, const V& v) {
+  if constexpr (sizeof(V) == 16)
+    __stcs(reinterpret_cast<float4*>(p), reinterpret_cast<const float4&>(v));
+  else
+    __stcs(reinterpret_cast<float2*>(p), reinterpret_cast<const float2&>(v));
+}
+
 // ---------------------------------------------------------------------------
 // Elementwise kernels
 // ---------------------------------------------------------------------------
 
-// data[i] = conj?(src[i]) * factor   (normalize, copies)
-template <typename T>
-__global__ void k_scale_copy(const typename Cx<T>::type* src, typename Cx<T>::type* dst, int64_t n,
-                             T factor, int conj) {
+// dst[i] = conj?(src[i]) * factor   (normalize, copies); src may be dst.
+// HBM bound: blocks of kScaleUnroll x 256 vectors of VW elements (16 bytes
+// where both buffers start on 16), all loads issued before the first store,
+// both streaming.  Measured on B200, 384^3 complex64 in place:
+// 165 -> 134 us, 6.75 TB/s (one 8-byte element a step of a grid-stride loop
+// before).
+constexpr int kScaleUnroll = 4;
+template <typename T, int VW>
+__global__ void __launch_bounds__(256)
+    k_scale_copy(const typename Cx<T>::type* src, typename Cx<T>::type* dst, int64_t n, T fx, T fy) {
   using C = typename Cx<T>::type;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    C x = src[i];
-    x.x *= factor;
-    x.y *= factor;
-    if (conj) x.y = -x.y;
-    dst[i] = x;
+  using V = MixChunk<C, VW>;
+  const int64_t nv = n / VW;
+  const int64_t i0 = (int64_t)blockIdx.x * (256 * kScaleUnroll) + threadIdx.x;
+  V x[kScaleUnroll];
+#pragma unroll
+  for (int u = 0; u < kScaleUnroll; ++u)
+    if (i0 + u * 256 < nv) x[u] = ld_vec(reinterpret_cast<const V*>(src) + i0 + u * 256);
+#pragma unroll
+  for (int u = 0; u < kScaleUnroll; ++u) {
+    if (i0 + u * 256 >= nv) continue;
+#pragma unroll
+    for (int k = 0; k < VW; ++k) x[u].v[k] = C{x[u].v[k].x * fx, x[u].v[k].y * fy};
+    st_vec(reinterpret_cast<V*>(dst) + i0 + u * 256, x[u]);
+  }
+  if (VW > 1 && blockIdx.x == 0 && threadIdx.x < n - nv * VW) {
+    const int64_t i = nv * VW + threadIdx.x;
+    dst[i] = C{src[i].x * fx, src[i].y * fy};
   }
 }
 

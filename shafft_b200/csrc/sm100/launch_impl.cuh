@@ -541,7 +541,18 @@ cudaError_t Launch<T>::pass(const PassGeom& g, const C* in, C* out, const PassTa
 template <typename T>
 cudaError_t Launch<T>::scale_copy(const C* src, C* dst, int64_t n, T factor, int conj,
                                   cudaStream_t s) {
-  k_scale_copy<T><<<ew_grid(n), 256, 0, s>>>(src, dst, n, factor, conj);
+  if (n <= 0) return cudaSuccess;
+  constexpr int VW = 16 / (int)sizeof(C);
+  const T fy = conj ? -factor : factor;
+  const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
+  const int64_t per = 256 * kScaleUnroll * (vec ? VW : 1);
+  const unsigned grid = (unsigned)((n + per - 1) / per);
+  if (vec)
+    k_scale_copy<T, VW><<<grid, 256, 0, s>>>(src, dst, n, factor, fy);
+  else if constexpr (VW > 1)
+    k_scale_copy<T, 1><<<grid, 256, 0, s>>>(src, dst, n, factor, fy);
+  else
+    return cudaErrorMisalignedAddress;  // a 16-byte element that is not on 16 bytes
   return cudaGetLastError();
 }
 
