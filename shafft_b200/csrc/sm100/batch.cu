@@ -66,6 +66,7 @@ constexpr int64_t kBatchDirectMax = 362;  // the plans' direct-DFT range (plan.c
 // defaults of axes it has not timed
 constexpr int kBatchRowWMax = 256, kBatchColWMax = 64;
 constexpr int kBatchRowWDefault = 256, kBatchColWDefault = 64;
+constexpr int64_t kBatchTile = 4096;  // points of a tile, where an axis allows it
 
 // 16-byte aligned so that a warp copies each slot's PassGeom as int4s
 template <typename C>
@@ -113,8 +114,12 @@ __device__ __forceinline__ int ticket_slot(long long t, const int* tslot, const 
 // Thread 0 claims a ticket and finds its slot (a table lookup), waits for the
 // slot's previous pass, and warp 0 copies the slot's geometry to shared
 // memory with all its lanes.
-// complex64: at most 80 registers so that three CTAs share an SM (the tiles
-// are latency-bound; 116 registers allowed only two); complex128 unbounded
+// complex64: at most 80 registers, i.e. 768 threads an SM (the tiles are
+// latency-bound; 116 registers allowed only 512).  As six CTAs of 128 threads
+// and 4096-point tiles, or three of 256 where a long axis needs a larger tile
+// (the choice is made once a batch): 512 uneven transforms take 3.21 ms in
+// the first form, 3.49 in the second with 8192-point tiles, 3.40 as four CTAs
+// of 192, 3.65 as twelve of 64 (B200).  complex128 unbounded.
 template <typename T>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1)
     k_fft_batch(const SlotDesc<typename Cx<T>::type>* slots, const int64_t* start, const int* tslot, int nslots,
@@ -243,6 +248,7 @@ struct shafft_sm100_batch_s {
   int64_t alg_bytes = 0;
   size_t smem = 0;
   unsigned grid = 0;
+  int threads = 0;  // block size
   // device memory
   unsigned char* d_tables = nullptr;  // twiddle + digit tables per distinct length
   void* d_slots = nullptr;
@@ -440,14 +446,14 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
       int W;
       if (row) {
         // tile widths are powers of two (the tile walks columns by mask and shift)
-        const int def = pow2_floor((int)std::min<int64_t>(kBatchRowWDefault, std::max<int64_t>(1, 8192 / L)));
+        const int def = pow2_floor((int)std::min<int64_t>(kBatchRowWDefault, std::max<int64_t>(1, kBatchTile / L)));
         W = tune_width<T>(L, true, O, def, es, autotune);
         g.ext[0] = O;
         g.sin[0] = g.sout[0] = L;
         g.ext[1] = g.ext[2] = g.ext[3] = 1;
         g.sn_in = g.sk_out = 1;
       } else {
-        const int def = pow2_floor((int)std::min<int64_t>(kBatchColWDefault, std::max<int64_t>(1, 8192 / L)));
+        const int def = pow2_floor((int)std::min<int64_t>(kBatchColWDefault, std::max<int64_t>(1, kBatchTile / L)));
         W = tune_width<T>(L, false, I, def, es, autotune);
         g.ext[0] = I;
         g.sin[0] = g.sout[0] = 1;
@@ -601,7 +607,9 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
   int dev = 0, sms = 148, per = 1;
   BCUDA(cudaGetDevice(&dev));
   BCUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  BCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fft_batch<T>, kThreads, b->smem));
+  // 128 threads where shared memory leaves room for the six CTAs that need
+  b->threads = 6 * (b->smem + 1024) <= (227 << 10) ? 128 : kThreads;
+  BCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fft_batch<T>, b->threads, b->smem));
   b->grid = (unsigned)(sms * std::max(per, 1));
   char buf[256];
   snprintf(buf, sizeof(buf),
@@ -617,7 +625,7 @@ template <typename T>
 int batch_launch(shafft_sm100_batch_s* b, int conj, double scale, cudaStream_t s) {
   using C = typename Vec2<T>::type;
   BCUDA(cudaMemsetAsync(b->d_ctl, 0, sizeof(int) * (4 + b->nslots), s));
-  k_fft_batch<T><<<b->grid, kThreads, b->smem, s>>>(
+  k_fft_batch<T><<<b->grid, b->threads, b->smem, s>>>(
       reinterpret_cast<const SlotDesc<C>*>(b->d_slots), b->d_start, b->d_tslot, b->nslots,
       reinterpret_cast<C* const*>(b->d_src), reinterpret_cast<C* const*>(b->d_dst), b->d_ctl + 4,
       reinterpret_cast<unsigned long long*>(b->d_ctl), b->d_ctl + 2, conj, scale, b->wait_limit);
