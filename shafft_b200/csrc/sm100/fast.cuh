@@ -476,6 +476,7 @@ template <typename T, int L, int R0, int R1, int R2, int NT, bool IN_ROW, int EX
 __global__ void __launch_bounds__(NT)
     k_fft_fast(const __grid_constant__ PassGeom g, const typename Cx<T>::type* in,
                typename Cx<T>::type* out, const __grid_constant__ PassTables<typename Cx<T>::type> tb) {
+  chain_begin();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   fast_tile<T, L, R0, R1, R2, NT, IN_ROW, LD_STREAM, ST_STREAM, false, false, EXT>(
       g, in, out, tb, blockIdx.x, reinterpret_cast<float4*>(smem_raw));
@@ -538,6 +539,7 @@ __global__ void __launch_bounds__(NT, fast_pf_min_blocks<T, L>())
     k_fft_fast_pf(const __grid_constant__ PassGeom g, const typename Cx<T>::type* in,
                   typename Cx<T>::type* out, const __grid_constant__ PassTables<typename Cx<T>::type> tb,
                   int64_t ahead, int bulk) {
+  chain_begin();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float4* sm = reinterpret_cast<float4*>(smem_raw);
   const int64_t nt = (int64_t)blockIdx.x + ahead;

@@ -204,6 +204,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads)
     k_fft_direct(const __grid_constant__ PassGeom g, const typename Cx<T>::type* in,
                  typename Cx<T>::type* out, const __grid_constant__ PassTables<typename Cx<T>::type> tb) {
+  chain_begin();
   using C = typename Cx<T>::type;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   C* sm = reinterpret_cast<C*>(smem_raw);
@@ -246,6 +247,7 @@ constexpr int kScaleUnroll = 4;
 template <typename T, int VW>
 __global__ void __launch_bounds__(256)
     k_scale_copy(const typename Cx<T>::type* src, typename Cx<T>::type* dst, int64_t n, T fx, T fy) {
+  chain_begin();
   using C = typename Cx<T>::type;
   using V = MixChunk<C, VW>;
   const int64_t nv = n / VW;

@@ -227,11 +227,8 @@ template <typename T, int L, int A, int B, int C_, int NT, int X>
 static cudaError_t fast_ext_launch(bool in_row, unsigned grid, const PassGeom& g, const typename Vec2<T>::type* in,
                                    typename Vec2<T>::type* out, const PassTables<typename Vec2<T>::type>& tb,
                                    cudaStream_t s) {
-  if (in_row)
-    k_fft_fast<T, L, A, B, C_, NT, true, X><<<grid, NT, L * 128, s>>>(g, in, out, tb);
-  else
-    k_fft_fast<T, L, A, B, C_, NT, false, X><<<grid, NT, L * 128, s>>>(g, in, out, tb);
-  return cudaGetLastError();
+  return launch_chained(in_row ? k_fft_fast<T, L, A, B, C_, NT, true, X> : k_fft_fast<T, L, A, B, C_, NT, false, X>,
+                        grid, NT, L * 128, s, g, in, out, tb);
 }
 template <typename T, int L, int A, int B, int C_, int NT>
 struct FastExt {
@@ -321,9 +318,10 @@ struct FastPf {
     }
     return cudaSuccess;
   }
-  // false: not taken (switched off, or no prefetching instantiation for L)
+  // false: not taken (switched off, or no prefetching instantiation for L); else *e is the launch's result
   static bool launch(bool in_row, unsigned grid, const PassGeom& g, const typename Vec2<T>::type* in,
-                     typename Vec2<T>::type* out, const PassTables<typename Vec2<T>::type>& tb, cudaStream_t s) {
+                     typename Vec2<T>::type* out, const PassTables<typename Vec2<T>::type>& tb, cudaStream_t s,
+                     cudaError_t* e) {
     if constexpr (kOn) {
       const int q = prefetch_quarters(in_row);
       const bool fetch = !in_row && col_fetch_256();
@@ -333,12 +331,13 @@ struct FastPf {
       const int64_t resident = (int64_t)sm_count() * fast_pf_min_blocks<T, L>();
       const int64_t ahead = q == 0 ? 0 : std::max<int64_t>(1, resident * q / 4);
       if (in_row)
-        k_fft_fast_pf<T, L, A, B, C_, NT, true>
-            <<<grid, NT, L * 128, s>>>(g, in, out, tb, ahead, bulk_prefetch());
+        *e = launch_chained(k_fft_fast_pf<T, L, A, B, C_, NT, true>, grid, NT, L * 128, s, g, in, out, tb, ahead,
+                            bulk_prefetch());
       else if (fetch)
-        k_fft_fast_pf<T, L, A, B, C_, NT, false, 256><<<grid, NT, L * 128, s>>>(g, in, out, tb, ahead, 0);
+        *e = launch_chained(k_fft_fast_pf<T, L, A, B, C_, NT, false, 256>, grid, NT, L * 128, s, g, in, out, tb, ahead,
+                            0);
       else
-        k_fft_fast_pf<T, L, A, B, C_, NT, false><<<grid, NT, L * 128, s>>>(g, in, out, tb, ahead, 0);
+        *e = launch_chained(k_fft_fast_pf<T, L, A, B, C_, NT, false>, grid, NT, L * 128, s, g, in, out, tb, ahead, 0);
       return true;
     }
     return false;
@@ -458,12 +457,10 @@ static cudaError_t fast_attr_all();
 #define SHAFFT_CASE_FAST(L_, A, B, C_, NT)                                                       \
   case L_:                                                                                       \
     if (g.bs_mode || g.map_mode) return FastExt<TYPE_, L_, A, B, C_, NT>::launch(in_row, grid, g, in, out, tb, s); \
-    if (FastPf<TYPE_, L_, A, B, C_, NT>::launch(in_row, grid, g, in, out, tb, s)) return cudaGetLastError(); \
-    if (in_row)                                                                                  \
-      k_fft_fast<TYPE_, L_, A, B, C_, NT, true><<<grid, NT, L_ * 128, s>>>(g, in, out, tb);      \
-    else                                                                                         \
-      k_fft_fast<TYPE_, L_, A, B, C_, NT, false><<<grid, NT, L_ * 128, s>>>(g, in, out, tb);     \
-    return cudaGetLastError();
+    if (cudaError_t e; FastPf<TYPE_, L_, A, B, C_, NT>::launch(in_row, grid, g, in, out, tb, s, &e)) return e; \
+    return launch_chained(in_row ? k_fft_fast<TYPE_, L_, A, B, C_, NT, true>                     \
+                                 : k_fft_fast<TYPE_, L_, A, B, C_, NT, false>,                   \
+                          grid, NT, L_ * 128, s, g, in, out, tb);
 #define SHAFFT_CASE_PLANE(L_, A, B, C_, NT)                                                      \
   case L_:                                                                                       \
     return launch_flow<TYPE_>(k_fft_plane_flow<TYPE_, L_, A, B, C_, NT>, NT, L_ * 128 + 128, gx, \
@@ -517,25 +514,19 @@ cudaError_t Launch<T>::pass(const PassGeom& g, const C* in, C* out, const PassTa
   const size_t smem = pass_smem(g, sizeof(C));
   if (g.nst == 0) {
     const int64_t grid = std::min<int64_t>(g.ntiles, 148 * 64);
-    k_fft_direct<T><<<(unsigned)grid, g.threads, smem, s>>>(g, in, out, tb);
-    return cudaGetLastError();
+    return launch_chained(k_fft_direct<T>, (unsigned)grid, g.threads, smem, s, g, in, out, tb);
   }
   constexpr int VW = sizeof(T) == 4 ? 2 : 1;
   const unsigned grid = (unsigned)std::min<int64_t>(g.ntiles, 0x7fffffff);
-  if (VW == 2 && g.W == 1) {
-    k_fft_mix<T, 1, true><<<grid, g.threads, smem, s>>>(g, in, out, tb);
-    return cudaGetLastError();
-  }
+  if (VW == 2 && g.W == 1) return launch_chained(k_fft_mix<T, 1, true>, grid, g.threads, smem, s, g, in, out, tb);
   // The unpermuted tile spares a few instructions an access where column tiles
   // allow it; below two waves of tiles one kernel for every pass is better
   // (its code stays in the instruction caches from pass to pass: 8575 points
   // complex64 9.1 us, 12.5 us with the two kernels in turn).
   const int nc = g.W / VW;
-  if (g.in_row || g.out_row || nc < 8 || g.ntiles < 2 * 3 * 148)
-    k_fft_mix<T, VW, true><<<grid, g.threads, smem, s>>>(g, in, out, tb);
-  else
-    k_fft_mix<T, VW, false><<<grid, g.threads, smem, s>>>(g, in, out, tb);
-  return cudaGetLastError();
+  const bool permuted = g.in_row || g.out_row || nc < 8 || g.ntiles < 2 * 3 * 148;
+  return launch_chained(permuted ? k_fft_mix<T, VW, true> : k_fft_mix<T, VW, false>, grid, g.threads, smem, s, g, in,
+                        out, tb);
 }
 
 template <typename T>
@@ -548,12 +539,9 @@ cudaError_t Launch<T>::scale_copy(const C* src, C* dst, int64_t n, T factor, int
   const int64_t per = 256 * kScaleUnroll * (vec ? VW : 1);
   const unsigned grid = (unsigned)((n + per - 1) / per);
   if (vec)
-    k_scale_copy<T, VW><<<grid, 256, 0, s>>>(src, dst, n, factor, fy);
-  else if constexpr (VW > 1)
-    k_scale_copy<T, 1><<<grid, 256, 0, s>>>(src, dst, n, factor, fy);
-  else
-    return cudaErrorMisalignedAddress;  // a 16-byte element that is not on 16 bytes
-  return cudaGetLastError();
+    return launch_chained(k_scale_copy<T, VW>, grid, 256, 0, s, src, dst, n, factor, fy);
+  if constexpr (VW > 1) return launch_chained(k_scale_copy<T, 1>, grid, 256, 0, s, src, dst, n, factor, fy);
+  return cudaErrorMisalignedAddress;  // a 16-byte element that is not on 16 bytes
 }
 
 template <typename T>

@@ -370,6 +370,7 @@ template <typename T, int VW, bool SWZ>
 __global__ void __launch_bounds__(kThreads, 3)
     k_fft_mix(const __grid_constant__ PassGeom g, const typename Cx<T>::type* in, typename Cx<T>::type* out,
               const __grid_constant__ PassTables<typename Cx<T>::type> tb) {
+  chain_begin();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   for (int64_t tile = blockIdx.x; tile < g.ntiles; tile += gridDim.x) {
     if (tile != blockIdx.x) __syncthreads();  // the previous tile is read out

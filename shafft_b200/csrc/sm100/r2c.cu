@@ -99,6 +99,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     k_r2c_untangle(const typename Cx<T>::type* Z, typename Cx<T>::type* X, int64_t rows, int64_t H, int64_t chunks, int logG,
                    const typename Cx<T>::type* tw, T scale, const RDims d) {
+  chain_begin();
   using C = typename Cx<T>::type;
   int64_t r, mr, k0;
   if (!rc_item(d, rows, chunks, logG, r, mr, k0)) return;
@@ -140,6 +141,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     k_c2r_tangle(const typename Cx<T>::type* X, typename Cx<T>::type* Z, int64_t rows, int64_t H, int64_t chunks, int logG,
                  const typename Cx<T>::type* tw, const RDims d) {
+  chain_begin();
   using C = typename Cx<T>::type;
   int64_t r, mr, k0;
   if (!rc_item(d, rows, chunks, logG, r, mr, k0)) return;
@@ -299,17 +301,19 @@ int shafft_sm100_execute_r2c(shafft_sm100_rplan p, void* real_in, void* spec_out
   const int rc = shafft_sm100_execute(p->full, real_in, p->a, 0, 1.0, stream);
   if (rc) return rc;
   const RcShape g = rc_shape(p->rows, p->H);
+  cudaError_t e;
   if (p->precision)
-    k_r2c_untangle<double><<<g.grid, 256, 0, s>>>(
+    e = launch_chained(
+        k_r2c_untangle<double>, g.grid, 256, 0, s,
         reinterpret_cast<const double2*>(p->a),
         reinterpret_cast<double2*>(spec_out), p->rows, p->H, g.chunks, g.logG,
         reinterpret_cast<const double2*>(p->tw), scale, p->dims);
   else
-    k_r2c_untangle<float><<<g.grid, 256, 0, s>>>(
+    e = launch_chained(
+        k_r2c_untangle<float>, g.grid, 256, 0, s,
         reinterpret_cast<const float2*>(p->a),
         reinterpret_cast<float2*>(spec_out), p->rows, p->H, g.chunks, g.logG,
         reinterpret_cast<const float2*>(p->tw), (float)scale, p->dims);
-  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return rfail(SHAFFT_SM100_ECUDA, "untangle launch: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -319,15 +323,17 @@ int shafft_sm100_execute_c2r(shafft_sm100_rplan p, void* spec_in, void* real_out
   if (real_out == spec_in) return rfail(SHAFFT_SM100_EINVAL, "input and output must be distinct buffers");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const RcShape g = rc_shape(p->rows, p->H);
+  cudaError_t e;
   if (p->precision)
-    k_c2r_tangle<double><<<g.grid, 256, 0, s>>>(
+    e = launch_chained(
+        k_c2r_tangle<double>, g.grid, 256, 0, s,
         reinterpret_cast<const double2*>(spec_in), reinterpret_cast<double2*>(p->a), p->rows, p->H, g.chunks, g.logG,
         reinterpret_cast<const double2*>(p->tw), p->dims);
   else
-    k_c2r_tangle<float><<<g.grid, 256, 0, s>>>(
+    e = launch_chained(
+        k_c2r_tangle<float>, g.grid, 256, 0, s,
         reinterpret_cast<const float2*>(spec_in), reinterpret_cast<float2*>(p->a), p->rows, p->H, g.chunks, g.logG,
         reinterpret_cast<const float2*>(p->tw), p->dims);
-  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return rfail(SHAFFT_SM100_ECUDA, "tangle launch: %s", cudaGetErrorString(e));
   return shafft_sm100_execute(p->full, p->a, real_out, 1, scale, stream);
 }
