@@ -497,7 +497,7 @@ struct Planner {
   }
 
   // choose 2- or 3-factor split of a smooth L; returns empty if impossible
-  std::vector<int> split(int64_t L, int64_t I) const {
+  std::vector<int> split(int64_t L, int64_t I, bool in_bluestein) const {
     // SHAFFT_SM100_FACTORS="a,b[,c]": factor list for an axis of length a*b*c
     // (planning experiments); ignored for any other length
     if (const char* e = getenv("SHAFFT_SM100_FACTORS")) {
@@ -512,21 +512,26 @@ struct Planner {
       }
       if (prod == L && f.size() >= 2 && f.size() <= 3) return f;
     }
-    // Prefer factors that all have a specialised pass, the fewest passes, and
-    // for complex64 among those the most balanced split (largest smallest
-    // factor; ties to the larger last factor).  Balanced splits keep tiles small enough for
-    // several CTAs per SM: measured on B200, 2^24 = 256*256*256 runs 17%
-    // faster than 16*1024*1024.
+    // Factors that all have a specialised pass, if there are such.  Two short
+    // ones; else the three most balanced (largest smallest factor; ties to the
+    // larger last factor): three passes over tiles that leave room for several
+    // CTAs per SM beat two over 64 and 128 KiB tiles.  B200, device time, two
+    // and three factors: complex64 2^17 256*512 10.2 / 10.7 us, 2^19 512*1024
+    // 16.1 / 64*64*128 11.8, 2^20 1024*1024 19.9 / 64*64*256 14.4; complex128
+    // 2^15 128*256 7.8 / 8.0, 2^16 256*256 10.4 / 32*32*64 8.9, 2^17 11.6 /
+    // 9.4.  (512*512 stays in both types, the shortest plan of the 512-point
+    // kernels' variants, although three factors take 9.7 and 10.1 us for 12.5
+    // and 12.3.)  complex128 from 32 MB on takes the largest last factor
+    // instead (2^24: 64*512*512 342 us, 256^3 362; equal at 2^22 and 2^23).
     {
       const int64_t fl[] = {1024, 512, 256, 128, 64, 32, 16};
       std::vector<int> best2, best3;
       int64_t m2 = 0, m3 = 0;
+      const bool first_only =
+          balanced < 0 ? precision != 0 && (size_t)L * (size_t)I * elem >= (size_t)1 << 25 : balanced == 0;
       for (int64_t d : fl) {
         if (L % d || !fast_len(d)) continue;
         const int64_t c = L / d;
-        // complex128 (tiles twice the bytes): the largest last factor wins
-        // instead (2^24 = 64*512*512: 0.78 ms vs 0.87 ms for 256^3)
-        const bool first_only = balanced < 0 ? precision != 0 : balanced == 0;
         if (fast_len(c) && c >= 16 && std::min(c, d) > m2 && !(first_only && m2 > 0)) {
           m2 = std::min(c, d);
           best2 = {(int)c, (int)d};
@@ -540,35 +545,63 @@ struct Planner {
           }
         }
       }
-      if (!best2.empty()) return best2;
+      const int64_t two_max = precision && !in_bluestein ? 1 << 15 : 1 << 18;
+      if (!best2.empty() && (balanced == 0 || best3.empty() || L <= two_max || best2[0] * best2[1] == 1 << 18))
+        return best2;
       if (!best3.empty()) return best3;
     }
     const int max_last = (I == 1) ? lim.max_row : lim.max_col;
-    std::vector<int> best;
-    // 2 factors, as balanced as the pass limits allow (smaller one first):
-    // 1,488,375 = 1215*1225 measured 17% faster than 375*3969
+    // Generic passes: two factors, as balanced as the pass limits allow
+    // (1,488,375 = 1215*1225 measured 17% faster than 375*3969), an odd last
+    // one (complex64 rows on 8 bytes) counting as a sixth less balanced:
+    // 3,000,000 = 1875*1600 55 us, 1600*1875 71 us.
+    std::vector<int> pair;
     {
-      int64_t bm = 0;
+      double bm = 0;
       for (int64_t d = std::min<int64_t>(L, max_last); d >= 2; --d) {
         if (L % d) continue;
         const int64_t c = L / d;
-        if (c < 2 || c > lim.max_col || std::min(c, d) <= bm) continue;
-        bm = std::min(c, d);
-        best = {(int)c, (int)d};
+        if (c < 2 || c > lim.max_col) continue;
+        const double m = (double)std::min(c, d) * (precision == 0 && d % 2 && balanced != 0 ? 5.0 / 6 : 1.0);
+        if (m <= bm) continue;
+        bm = m;
+        pair = {(int)c, (int)d};
         if (balanced == 0) break;  // the largest last factor that fits
       }
     }
-    if (!best.empty()) return best;
-    for (int64_t d = std::min<int64_t>(L, max_last); d >= 2; --d) {
-      if (L % d) continue;
-      int64_t c = L / d;
-      // split c into two column factors as balanced as possible
-      int64_t bestf = -1;
-      for (int64_t f = 2; f * f <= c; ++f)
-        if (c % f == 0 && f <= lim.max_col && c / f <= lim.max_col) bestf = f;
-      if (bestf > 0) return {(int)(c / bestf), (int)bestf, (int)d};
+    // Three factors where the longer of two leaves a 64 KiB tile only narrow
+    // rows.  B200, two and three: complex64 1,488,375 36.8 / 37.7 us, 5,760,000
+    // (2000*2880) 91.7 / 94.8; complex128 1000*1000 23.8 / 32.1, 1,488,375 49.4
+    // / 45.9, 5,760,000 217 / 171.
+    const int two_longest = precision ? 1024 : 3072;
+    if (!pair.empty() && (balanced == 0 || std::max(pair[0], pair[1]) <= two_longest)) return pair;
+    // The smallest largest factor, ordered so that the strides of the earlier
+    // passes are whole 128-byte lines where that can be (else counting as 6 or
+    // 12% larger): 12,000,000 = 192*250*250 199 us, 250*250*192 169 us;
+    // before, for want of two factors, 60*50*4000, 234 us.
+    std::vector<int> triple;
+    double least = 0;
+    for (int64_t a = 2; a * a * a <= L && a <= lim.max_col; ++a) {
+      if (L % a) continue;
+      for (int64_t f = a; f * f <= L / a && f <= lim.max_col; ++f) {
+        const int64_t d = L / a / f;
+        if ((L / a) % f || d > std::min(max_last, lim.max_col)) continue;
+        int64_t t[3] = {a, f, d};
+        for (int i = 2; i >= 0; --i)
+          if (t[i] % 16 == 0) {
+            std::rotate(t + i, t + i + 1, t + 3);
+            break;
+          }
+        const double m = (double)d * (t[2] % 16 == 0 ? 1.0 : t[1] * t[2] % 16 == 0 ? 1.06 : 1.12);
+        if (triple.empty() || m < least) {
+          least = m;
+          triple = {(int)t[0], (int)t[1], (int)t[2]};
+        }
+      }
     }
-    return {};
+    const int longest = triple.empty() ? 0 : *std::max_element(triple.begin(), triple.end());
+    if (!pair.empty() && (triple.empty() || longest > 512)) return pair;
+    return triple;
   }
 
   // global decimation-in-frequency over the factors Ls
@@ -750,7 +783,7 @@ struct Planner {
       return 0;
     }
     if (is_smooth(L)) {
-      std::vector<int> f = split(L, I);
+      std::vector<int> f = split(L, I, in_bluestein);
       if (!f.empty()) {
         // the last pass is out of place: it lands in other(x) where x is the
         // buffer the in-place passes used

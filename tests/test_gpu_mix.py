@@ -23,6 +23,8 @@ SHAPES = [(r, r) for r in range(2, 14)] + [          # one stage, rows and colum
     (2048, 6), (6, 2048), (1728, 17), (169, 121),   # narrow column tiles; odd extents
     (35, 27, 45), (3, 40, 33), (60, 50, 2), (1, 90, 1), (99, 64, 31 * 2), (384, 7, 18),
     (5, 12, 16), (1200, 1215),                       # long axes in both directions
+    (1 << 13,), (1 << 16,), (1 << 18,), (1 << 19,),  # two and three specialised factors
+    (13 ** 5,), (1215000,), (3, 5000, 7), (6561, 20),  # two and three generic ones, rows and columns
 ]
 
 
