@@ -78,7 +78,17 @@ template <>
 __device__ __forceinline__ float2 ld_stream<float2>(const float2* p) { return __ldcs(p); }
 template <>
 __device__ __forceinline__ double2 ld_stream<double2>(const double2* p) { return __ldcs(p); }
-__device__ __forceinline__ float4 ld_chunk(const void* p) { return __ldcs(reinterpret_cast<const float4*>(p)); }
+// Column tiles read each line once, whole: without a place in L1, which the
+// tiles leave little of and loads in flight need (B200, 512^3 complex64 column
+// pass 433 -> 419 us, 2^24 first pass 66 -> 64; row tiles keep ldcs: 128-point
+// complex128 rows 46 us, 48 without).
+__device__ __forceinline__ float4 ld_chunk(const void* p) {
+  float4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p));
+  return v;
+}
 // The same load asking L2 to fetch the whole 256-byte block around the line
 // (the neighbouring column tile's line comes with it).
 __device__ __forceinline__ float4 ld_chunk_256(const void* p) {
@@ -470,10 +480,21 @@ __device__ __forceinline__ void fast_tile(const PassGeom& g, const typename Cx<T
   fast_finish<T, L, R0, R1, R2, NT, IN_ROW, LDP_, STP_, DISCARD_, SMEM_A, EXT>(g, in, out, tb, tile, sm, R, pol);
 }
 
+// Resident CTAs per SM a pass is compiled for.  complex128 of 256 and 512
+// points would take 86 to 88 registers, one CTA fewer than shared memory
+// allows: bounded at 512 (512 x 512 x 64: 114 -> 107 and 119 -> 113 us a
+// pass), not at 256, where the sixth CTA leaves too little L1 for the loads in
+// flight (101 -> 121 us).  0: not bounded; the others come out at their
+// occupancy by themselves.
+template <typename T, int L>
+constexpr int fast_min_blocks() {
+  return sizeof(T) == 8 && L == 512 ? 3 : 0;
+}
+
 // EXT: the plain pass (0), or the instantiation with the fused Bluestein
 // loads and stores (EXT_BS) or with an exchange block map (EXT_MAP)
 template <typename T, int L, int R0, int R1, int R2, int NT, bool IN_ROW, int EXT = 0>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, fast_min_blocks<T, L>())
     k_fft_fast(const __grid_constant__ PassGeom g, const typename Cx<T>::type* in,
                typename Cx<T>::type* out, const __grid_constant__ PassTables<typename Cx<T>::type> tb) {
   chain_begin();
