@@ -1123,7 +1123,8 @@ MixShape mix_shape(const PassGeom& g, size_t elem) {
     const double waves = (double)g.ntiles / (148.0 * ctas);
     const double rest = std::ceil((waves - std::floor(waves)) * ctas - 1e-9) / ctas;
     const double t =
-        (std::floor(waves) + (rest > 0 ? std::max(0.5, rest) : 0.0)) * ((double)g.L * g.W / busy + 6.0);
+        (std::floor(waves) + (rest > 0 ? std::max(0.5, rest) : 0.0)) * ((double)g.L * g.W / busy + 6.0) *
+        ((size_t)std::min<int64_t>(ctas, (g.ntiles + 147) / 148) * (smem + 1024) > (196 << 10) ? 1.2 : 1.0);
     if (best.time < 0 || t < best.time * 0.999) best = MixShape{nt, t};
   }
   return best;
