@@ -279,12 +279,12 @@ template <typename T>
 int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, int autotune) {
   const int maxw_smem = (int)std::max<int64_t>(1, (96 * 1024) / ((L + 1) * (int64_t)es));
   std::vector<int> cands;
-  // widest tiles: 256 for rows, 64 for columns (the synthetic column tensor
-  // has 64 columns), and at most 8192 points a tile
+  // tiles of a quarter of kBatchTile to kBatchTile points, 256 rows or 64
+  // columns (the width of the synthetic column tensor) at most
   const int wmax = row ? kBatchRowWMax : kBatchColWMax;
   for (int w = 1; w <= wmax; w *= 2) {
-    if (w > maxw_smem || (w > 1 && (int64_t)w * L > 8192)) break;
-    if (!row && w < 4 && ext0 >= 4) continue;
+    if (w > maxw_smem || (w > 1 && (int64_t)w * L > kBatchTile)) break;
+    if ((int64_t)w * L * 4 < kBatchTile && w < wmax && w < ext0) continue;
     if (w > 1 && w / 2 >= ext0) break;
     cands.push_back(w);
   }
@@ -352,6 +352,7 @@ int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, int 
     g.out_row = row ? 1 : 0;
     g.scale = 1.0;
     geom_derive(g, es);
+    g.threads = 6 * (pass_smem(g, es) + 1024) <= (227 << 10) ? 128 : kThreads;  // as the batch runs it
     float ms = 0;
     for (int rep = 0; rep < 4; ++rep) {
       cudaEventRecord(e0);
@@ -363,6 +364,9 @@ int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, int 
       if (rep > 0) ms += t;  // first run warms up
     }
     if (cudaGetLastError() != cudaSuccess) continue;
+    // in a batch each tile also costs its CTA a ticket (atomic, slot lookup,
+    // wait, geometry: about 2 us), which this launch does without
+    ms += 3 * 2e-3f * (float)g.ntiles / (148 * 6);
     if (ms < best_ms) {
       best_ms = ms;
       best = w;
@@ -468,10 +472,16 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
       W = std::max(1, std::min(W, cap));
       // radix passes work on 16-byte chunks: two complex64 columns
       if (g.nst > 0) W = std::max(W, sizeof(T) == 4 ? 2 : 1);
-      g.W = W;
-      g.logW = 0;
-      while ((1 << g.logW) < W) ++g.logW;
-      g.pitch = generic_pitch(W, row);
+      // narrower where that lets six CTAs share an SM (one large tile would set
+      // the whole batch's block size)
+      const int least = g.nst > 0 && sizeof(T) == 4 ? 2 : 1;
+      for (;; W /= 2) {
+        g.W = W;
+        g.logW = 0;
+        while ((1 << g.logW) < W) ++g.logW;
+        g.pitch = generic_pitch(W, row);
+        if (W <= least || L * W * 2 <= kBatchTile || 6 * (pass_smem(g, es) + 1024) <= (227 << 10)) break;
+      }
       g.tiles_w = (g.ext[0] + W - 1) / W;
       g.ntiles = g.tiles_w * g.ext[1] * g.ext[2] * g.ext[3];
       g.in_row = row ? 1 : 0;
