@@ -578,24 +578,29 @@ struct Planner {
     // The smallest largest factor, ordered so that the strides of the earlier
     // passes are whole 128-byte lines where that can be (else counting as 6 or
     // 12% larger): 12,000,000 = 192*250*250 199 us, 250*250*192 169 us;
-    // before, for want of two factors, 60*50*4000, 234 us.
+    // before, for want of two factors, 60*50*4000, 234 us.  Where no three fit
+    // a column pass, the longest one is the row pass of a contiguous axis
+    // (13^7 = 169*169*2197): six passes over a padded convolution otherwise.
     std::vector<int> triple;
     double least = 0;
-    for (int64_t a = 2; a * a * a <= L && a <= lim.max_col; ++a) {
-      if (L % a) continue;
-      for (int64_t f = a; f * f <= L / a && f <= lim.max_col; ++f) {
-        const int64_t d = L / a / f;
-        if ((L / a) % f || d > std::min(max_last, lim.max_col)) continue;
-        int64_t t[3] = {a, f, d};
-        for (int i = 2; i >= 0; --i)
-          if (t[i] % 16 == 0) {
-            std::rotate(t + i, t + i + 1, t + 3);
-            break;
+    for (const int64_t most : {std::min(max_last, lim.max_col), max_last}) {
+      if (!triple.empty()) break;
+      for (int64_t a = 2; a * a * a <= L && a <= lim.max_col; ++a) {
+        if (L % a) continue;
+        for (int64_t f = a; f * f <= L / a && f <= lim.max_col; ++f) {
+          const int64_t d = L / a / f;
+          if ((L / a) % f || d > most) continue;
+          int64_t t[3] = {a, f, d};
+          for (int i = 2; i >= 0 && d <= lim.max_col; --i)
+            if (t[i] % 16 == 0) {
+              std::rotate(t + i, t + i + 1, t + 3);
+              break;
+            }
+          const double m = (double)d * (t[2] % 16 == 0 ? 1.0 : t[1] * t[2] % 16 == 0 ? 1.06 : 1.12);
+          if (triple.empty() || m < least) {
+            least = m;
+            triple = {(int)t[0], (int)t[1], (int)t[2]};
           }
-        const double m = (double)d * (t[2] % 16 == 0 ? 1.0 : t[1] * t[2] % 16 == 0 ? 1.06 : 1.12);
-        if (triple.empty() || m < least) {
-          least = m;
-          triple = {(int)t[0], (int)t[1], (int)t[2]};
         }
       }
     }

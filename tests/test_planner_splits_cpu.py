@@ -1,0 +1,55 @@
+"""Host-only planner: how long axes are split (no GPU needed)."""
+import pytest
+
+from shafft_b200 import _sm100
+
+MAX_ROW, MAX_COL = 4096, 2048  # longest row and column pass
+
+
+def _smooth(limit, primes=(2, 3, 5, 7, 11, 13)):
+    out = [1]
+    for p in primes:
+        nxt = []
+        for v in out:
+            while v <= limit:
+                nxt.append(v)
+                v *= p
+        out = nxt
+    return out
+
+
+def _factors(n):
+    """Some split of n into at most three passes, the last one the longest."""
+    small = [a for a in range(1, MAX_COL + 1) if n % a == 0]
+    have = set(small)
+    for d in range(min(n, MAX_ROW), 0, -1):
+        if n % d:
+            continue
+        c = n // d
+        if any(c % a == 0 and c // a in have for a in small):
+            return True
+    return False
+
+
+@pytest.mark.parametrize("n,factors", [(13 ** 7, [169, 169, 2197]), (7 ** 10, [343, 343, 2401]),
+                                       (5 ** 13, [625, 625, 3125])])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_longest_factor_may_be_a_row_pass(n, factors, prec):
+    """Lengths whose three factors need one above the longest column pass: the
+    contiguous axis takes it as its row pass."""
+    steps = _sm100.plan_query([n], prec)["steps"]
+    assert [s["kind"] for s in steps] == ["pass"] * 3
+    assert [s["L"] for s in steps] == factors
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_smooth_lengths_with_factors_are_not_convolved(prec):
+    """Every 13-smooth length up to 2^31 that three passes can make is made of passes."""
+    for n in _smooth(1 << 31):
+        if n <= MAX_ROW:
+            continue
+        steps = _sm100.plan_query([n], prec)["steps"]
+        if all(s["kind"] == "pass" and not s["bs"] for s in steps):
+            assert len(steps) <= 3, n
+        else:
+            assert not _factors(n), n
