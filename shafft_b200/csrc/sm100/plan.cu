@@ -496,8 +496,10 @@ struct Planner {
     return true;
   }
 
-  // choose 2- or 3-factor split of a smooth L; returns empty if impossible
-  std::vector<int> split(int64_t L, int64_t I, bool in_bluestein) const {
+  // choose 2- or 3-factor split of a smooth L of a tensor (O, L, I); returns
+  // empty if impossible
+  std::vector<int> split(int64_t O, int64_t L, int64_t I, bool in_bluestein) const {
+    const int64_t points = O * L * I;
     // SHAFFT_SM100_FACTORS="a,b[,c]": factor list for an axis of length a*b*c
     // (planning experiments); ignored for any other length
     if (const char* e = getenv("SHAFFT_SM100_FACTORS")) {
@@ -517,37 +519,42 @@ struct Planner {
     // larger last factor): three passes over tiles that leave room for several
     // CTAs per SM beat two over 64 and 128 KiB tiles.  B200, device time, two
     // and three factors: complex64 2^17 256*512 10.2 / 10.7 us, 2^19 512*1024
-    // 16.1 / 64*64*128 11.8, 2^20 1024*1024 19.9 / 64*64*256 14.4; complex128
-    // 2^15 128*256 7.8 / 8.0, 2^16 256*256 10.4 / 32*32*64 8.9, 2^17 11.6 /
-    // 9.4.  (512*512 stays in both types, the shortest plan of the 512-point
-    // kernels' variants, although three factors take 9.7 and 10.1 us for 12.5
-    // and 12.3.)  complex128 from 32 MB on takes the largest last factor
-    // instead (2^24: 64*512*512 342 us, 256^3 362; equal at 2^22 and 2^23).
+    // 16.1 / 64*64*128 11.8, 2^20 1024*1024 19.9 / 64*64*256 14.4.  Between
+    // 2^16 and 2^18 complex128 takes three only where the whole tensor is too
+    // small for two to fill the chip: 2^17 256*512 / 32*32*128 alone 11.6 / 9.6,
+    // twice 22.2 / 21.1, 4 times 23.4 / 24.4, 64 times 168 / 183.  (2^18 stays
+    // 512*512, 64 complex128 rows 320 us, 64*64*64 347, although alone three
+    // take 9.7 and 10.1 us for 12.5 and 12.3.)
+    // complex128 pairs from 2^15 on take the largest last factor (64 rows of
+    // 2^15 64*512 / 128*256 36.9 / 40.2 us, alone equal; 2^16 128*512 / 256*256
+    // alone 8.8 / 10.3, 64 rows 71.3 / 75.7; 64 rows of 2^13 64*128 14.4 / 16*512
+    // 16.4), triples from 32 MB on (2^24: 64*512*512 342 us, 256^3 362; equal
+    // at 2^22 and 2^23).
     {
       const int64_t fl[] = {1024, 512, 256, 128, 64, 32, 16};
       std::vector<int> best2, best3;
       int64_t m2 = 0, m3 = 0;
-      const bool first_only =
+      const bool last2 = balanced < 0 ? precision != 0 && L >= 1 << 15 : balanced == 0;
+      const bool last3 =
           balanced < 0 ? precision != 0 && (size_t)L * (size_t)I * elem >= (size_t)1 << 25 : balanced == 0;
       for (int64_t d : fl) {
         if (L % d || !fast_len(d)) continue;
         const int64_t c = L / d;
-        if (fast_len(c) && c >= 16 && std::min(c, d) > m2 && !(first_only && m2 > 0)) {
+        if (fast_len(c) && c >= 16 && std::min(c, d) > m2 && !(last2 && m2 > 0)) {
           m2 = std::min(c, d);
           best2 = {(int)c, (int)d};
         }
         for (int64_t f : fl) {
           if (c % f || !fast_len(f) || !fast_len(c / f) || c / f < 16) continue;
           const int64_t mn = std::min(std::min(c / f, f), d);
-          if (mn > m3 && !(first_only && m3 > 0)) {
+          if (mn > m3 && !(last3 && m3 > 0)) {
             m3 = mn;
             best3 = {(int)(c / f), (int)f, (int)d};
           }
         }
       }
-      const int64_t two_max = precision && !in_bluestein ? 1 << 15 : 1 << 18;
-      if (!best2.empty() && (balanced == 0 || best3.empty() || L <= two_max || best2[0] * best2[1] == 1 << 18))
-        return best2;
+      const bool small = precision && !in_bluestein && L > 1 << 16 && L < 1 << 18 && points <= 1 << 18;
+      if (!best2.empty() && (balanced == 0 || best3.empty() || (L <= 1 << 18 && !small))) return best2;
       if (!best3.empty()) return best3;
     }
     const int max_last = (I == 1) ? lim.max_row : lim.max_col;
@@ -788,7 +795,7 @@ struct Planner {
       return 0;
     }
     if (is_smooth(L)) {
-      std::vector<int> f = split(L, I, in_bluestein);
+      std::vector<int> f = split(O, L, I, in_bluestein);
       if (!f.empty()) {
         // the last pass is out of place: it lands in other(x) where x is the
         // buffer the in-place passes used

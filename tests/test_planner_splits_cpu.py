@@ -53,3 +53,21 @@ def test_smooth_lengths_with_factors_are_not_convolved(prec):
             assert len(steps) <= 3, n
         else:
             assert not _factors(n), n
+
+
+@pytest.mark.parametrize("dims,factors", [
+    ((1 << 16,), [128, 512]), ((64, 1 << 15), [64, 512]), ((16, 1 << 16), [128, 512]), ((512, 1 << 16), [128, 512]),
+    ((64, 1 << 17), [256, 512]), ((1 << 17, 64), [256, 512]), ((1 << 17,), [32, 32, 128]), ((1 << 14,), [128, 128])])
+def test_complex128_axes_of_many_rows_take_two_passes(dims, factors):
+    """Three short factors are for a lone 2^17 signal; many of them take two
+    passes, the larger factor last."""
+    steps = _sm100.plan_query(list(dims), 1)["steps"]
+    lens = [s["L"] for s in steps]
+    n = len(factors)
+    assert any(lens[i:i + n] == factors for i in range(len(lens) - n + 1)), lens
+    assert len(lens) == n + len(dims) - 1
+
+
+def test_complex128_convolution_of_2p16():
+    steps = _sm100.plan_query([22651], 1)["steps"]
+    assert [s["L"] for s in steps if s["kind"] == "pass"] == [128, 512] * 2
