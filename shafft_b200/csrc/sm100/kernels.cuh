@@ -125,9 +125,12 @@ __device__ __forceinline__ void direct_sums(const PassGeom& g, const PassTables<
         if (k > half) continue;
         const T e = (k & 1) ? (T)-1 : (T)1;
         const T bx = x0.x + e * xh.x + P[i][c].x, by = x0.y + e * xh.y + P[i][c].y;
-        direct_put<T, C>(g, tb, out, C{bx - Q[i][c].y, by + Q[i][c].x}, k, w, at, scale);
-        if (k > 0 && 2 * k != L)
-          direct_put<T, C>(g, tb, out, C{bx + Q[i][c].y, by - Q[i][c].x}, L - k, w, at, scale);
+        // an output that is its own partner has no sine part: 0 times an
+        // infinite input would make it NaN
+        const bool own = k == 0 || 2 * k == L;
+        const C q = own ? C{0, 0} : Q[i][c];
+        direct_put<T, C>(g, tb, out, C{bx - q.y, by + q.x}, k, w, at, scale);
+        if (!own) direct_put<T, C>(g, tb, out, C{bx + q.y, by - q.x}, L - k, w, at, scale);
       }
     }
   }
