@@ -66,7 +66,14 @@ constexpr int64_t kBatchDirectMax = 362;  // the plans' direct-DFT range (plan.c
 // defaults of axes it has not timed
 constexpr int kBatchRowWMax = 256, kBatchColWMax = 64;
 constexpr int kBatchRowWDefault = 256, kBatchColWDefault = 64;
-constexpr int64_t kBatchTile = 4096;  // points of a tile, where an axis allows it
+
+// Block size of a batch, the CTAs of it that share an SM, and the points its
+// tiles hold where an axis allows it.
+struct BatchForm {
+  int threads, ctas;
+  int64_t tile;
+  bool fits(size_t smem) const { return ctas * (smem + 1024) <= (227 << 10); }
+};
 
 // 16-byte aligned so that a warp copies each slot's PassGeom as int4s
 template <typename C>
@@ -115,11 +122,8 @@ __device__ __forceinline__ int ticket_slot(long long t, const int* tslot, const 
 // slot's previous pass, and warp 0 copies the slot's geometry to shared
 // memory with all its lanes.
 // complex64: at most 80 registers, i.e. 768 threads an SM (the tiles are
-// latency-bound; 116 registers allowed only 512).  As six CTAs of 128 threads
-// and 4096-point tiles, or three of 256 where a long axis needs a larger tile
-// (the choice is made once a batch): 512 uneven transforms take 3.21 ms in
-// the first form, 3.49 in the second with 8192-point tiles, 3.40 as four CTAs
-// of 192, 3.65 as twelve of 64 (B200).  complex128 unbounded.
+// latency-bound; 116 registers allowed only 512); complex128 unbounded (168).
+// The shapes it is launched with: batch_form.
 template <typename T>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1)
     k_fft_batch(const SlotDesc<typename Cx<T>::type>* slots, const int64_t* start, const int* tslot, int nslots,
@@ -275,16 +279,42 @@ struct LenTab {
   size_t off_tw, off_p2k, off_k2p;
 };
 
+// complex64: six CTAs of 128 threads and 4096-point tiles, or three of 256
+// where a long axis needs a larger tile (the choice is made once a batch): 512
+// uneven transforms take 3.21 ms in the first form, 3.49 in the second with
+// 8192-point tiles, 3.40 as four CTAs of 192, 3.65 as twelve of 64 (B200).
+// complex128: three CTAs of 128 threads, as many as 168 registers leave room
+// for; every axis fits.  Against tiles of half the size and, from 2358 points
+// on, one CTA of 256: 64 x 96^3 1.63 -> 1.14 ms, 8 x 2048^2 1.35 -> 1.12, 16 x
+// 256 x 4096 0.81 -> 0.59.
 template <typename T>
-int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, int autotune) {
+BatchForm batch_form(const std::vector<int64_t>& dims) {
+  constexpr size_t es = 2 * sizeof(T);
+  if (es == 16) return BatchForm{128, 3, 4096};
+  const BatchForm form{128, 6, 4096};
+  for (const int64_t L : dims)
+    if (!form.fits(2 * L * es)) return BatchForm{kThreads, 3, 4096};  // narrowest tile of a radix pass
+  return form;
+}
+
+// Points of a tile of one axis.  complex128 direct-DFT tiles hold one column a
+// thread and are taken at half size: 24 transforms of two prime axes 76 us at
+// 2048 points, 119 at 4096.
+int64_t axis_tile(const BatchForm& form, bool direct, size_t es) {
+  return direct && es == 16 ? form.tile / 2 : form.tile;
+}
+
+template <typename T>
+int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, const BatchForm& form, int64_t tile,
+               int autotune) {
   const int maxw_smem = (int)std::max<int64_t>(1, (96 * 1024) / ((L + 1) * (int64_t)es));
   std::vector<int> cands;
-  // tiles of a quarter of kBatchTile to kBatchTile points, 256 rows or 64
-  // columns (the width of the synthetic column tensor) at most
+  // tiles of a quarter of `tile` to `tile` points, 256 rows or 64 columns (the
+  // width of the synthetic column tensor) at most
   const int wmax = row ? kBatchRowWMax : kBatchColWMax;
   for (int w = 1; w <= wmax; w *= 2) {
-    if (w > maxw_smem || (w > 1 && (int64_t)w * L > kBatchTile)) break;
-    if ((int64_t)w * L * 4 < kBatchTile && w < wmax && w < ext0) continue;
+    if (w > maxw_smem || (w > 1 && (int64_t)w * L > tile)) break;
+    if ((int64_t)w * L * 4 < tile && w < wmax && w < ext0) continue;
     if (w > 1 && w / 2 >= ext0) break;
     cands.push_back(w);
   }
@@ -352,7 +382,7 @@ int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, int 
     g.out_row = row ? 1 : 0;
     g.scale = 1.0;
     geom_derive(g, es);
-    g.threads = 6 * (pass_smem(g, es) + 1024) <= (227 << 10) ? 128 : kThreads;  // as the batch runs it
+    g.threads = form.threads;  // as the batch runs it
     float ms = 0;
     for (int rep = 0; rep < 4; ++rep) {
       cudaEventRecord(e0);
@@ -366,7 +396,7 @@ int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, int 
     if (cudaGetLastError() != cudaSuccess) continue;
     // in a batch each tile also costs its CTA a ticket (atomic, slot lookup,
     // wait, geometry: about 2 us), which this launch does without
-    ms += 3 * 2e-3f * (float)g.ntiles / (148 * 6);
+    ms += 3 * 2e-3f * (float)g.ntiles / (148 * form.ctas);
     if (ms < best_ms) {
       best_ms = ms;
       best = w;
@@ -424,6 +454,7 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
   std::vector<std::vector<HostSlot>> per_transform(b->count);
   std::map<int64_t, RadixPlan> plans;  // by axis length
   size_t maxsmem = 0;
+  const BatchForm form = batch_form<T>(b->dims);
   const int64_t* dp = b->dims.data();
   for (int t = 0; t < b->count; ++t) {
     const int nd = b->ndims[t];
@@ -447,18 +478,19 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
       g.nst = rp.n > 0 ? rp.n : 0;
       for (int s = 0; s < g.nst; ++s) g.rad[s] = rp.r[s];
       const bool row = (I == 1);
+      const int64_t tile = axis_tile(form, g.nst == 0, es);
       int W;
       if (row) {
         // tile widths are powers of two (the tile walks columns by mask and shift)
-        const int def = pow2_floor((int)std::min<int64_t>(kBatchRowWDefault, std::max<int64_t>(1, kBatchTile / L)));
-        W = tune_width<T>(L, true, O, def, es, autotune);
+        const int def = pow2_floor((int)std::min<int64_t>(kBatchRowWDefault, std::max<int64_t>(1, tile / L)));
+        W = tune_width<T>(L, true, O, def, es, form, tile, autotune);
         g.ext[0] = O;
         g.sin[0] = g.sout[0] = L;
         g.ext[1] = g.ext[2] = g.ext[3] = 1;
         g.sn_in = g.sk_out = 1;
       } else {
-        const int def = pow2_floor((int)std::min<int64_t>(kBatchColWDefault, std::max<int64_t>(1, kBatchTile / L)));
-        W = tune_width<T>(L, false, I, def, es, autotune);
+        const int def = pow2_floor((int)std::min<int64_t>(kBatchColWDefault, std::max<int64_t>(1, tile / L)));
+        W = tune_width<T>(L, false, I, def, es, form, tile, autotune);
         g.ext[0] = I;
         g.sin[0] = g.sout[0] = 1;
         g.ext[1] = O;
@@ -472,15 +504,15 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
       W = std::max(1, std::min(W, cap));
       // radix passes work on 16-byte chunks: two complex64 columns
       if (g.nst > 0) W = std::max(W, sizeof(T) == 4 ? 2 : 1);
-      // narrower where that lets six CTAs share an SM (one large tile would set
-      // the whole batch's block size)
+      // narrower where that lets the form's CTAs share an SM (one large tile
+      // would set the residency of the whole batch)
       const int least = g.nst > 0 && sizeof(T) == 4 ? 2 : 1;
       for (;; W /= 2) {
         g.W = W;
         g.logW = 0;
         while ((1 << g.logW) < W) ++g.logW;
         g.pitch = generic_pitch(W, row);
-        if (W <= least || L * W * 2 <= kBatchTile || 6 * (pass_smem(g, es) + 1024) <= (227 << 10)) break;
+        if (W <= least || L * W * 2 <= tile || form.fits(pass_smem(g, es))) break;
       }
       g.tiles_w = (g.ext[0] + W - 1) / W;
       g.ntiles = g.tiles_w * g.ext[1] * g.ext[2] * g.ext[3];
@@ -617,15 +649,14 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
   int dev = 0, sms = 148, per = 1;
   BCUDA(cudaGetDevice(&dev));
   BCUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // 128 threads where shared memory leaves room for the six CTAs that need
-  b->threads = 6 * (b->smem + 1024) <= (227 << 10) ? 128 : kThreads;
+  b->threads = form.threads;
   BCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fft_batch<T>, b->threads, b->smem));
   b->grid = (unsigned)(sms * std::max(per, 1));
   char buf[256];
   snprintf(buf, sizeof(buf),
            "{\"transforms\":%d,\"slots\":%d,\"tiles\":%lld,\"lengths\":%zu,\"smem\":%zu,\"grid\":%u,"
-           "\"alg_bytes\":%lld}",
-           b->count, b->nslots, (long long)b->tickets, lens.size(), b->smem, b->grid,
+           "\"threads\":%d,\"alg_bytes\":%lld}",
+           b->count, b->nslots, (long long)b->tickets, lens.size(), b->smem, b->grid, b->threads,
            (long long)b->alg_bytes);
   b->desc = buf;
   return 0;
