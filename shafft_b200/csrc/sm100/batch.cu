@@ -384,16 +384,17 @@ int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, cons
     geom_derive(g, es);
     g.threads = form.threads;  // as the batch runs it
     float ms = 0;
-    for (int rep = 0; rep < 4; ++rep) {
+    cudaError_t launched = cudaSuccess;
+    for (int rep = 0; rep < 4 && launched == cudaSuccess; ++rep) {
       cudaEventRecord(e0);
-      Launch<T>::pass(g, a, b, tb, nullptr);
+      launched = Launch<T>::pass(g, a, b, tb, nullptr);
       cudaEventRecord(e1);
       cudaEventSynchronize(e1);
       float t = 0;
       cudaEventElapsedTime(&t, e0, e1);
       if (rep > 0) ms += t;  // first run warms up
     }
-    if (cudaGetLastError() != cudaSuccess) continue;
+    if (cudaGetLastError() != cudaSuccess || launched != cudaSuccess) continue;
     // in a batch each tile also costs its CTA a ticket (atomic, slot lookup,
     // wait, geometry: about 2 us), which this launch does without
     ms += 3 * 2e-3f * (float)g.ntiles / (148 * form.ctas);

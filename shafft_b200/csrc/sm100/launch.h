@@ -78,7 +78,9 @@ cudaError_t launch_chained(void (*kernel)(Params...), unsigned grid, unsigned th
   cfg.stream = s;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not again by the next launch's check
+  return e;
 }
 
 template <typename T>
