@@ -1143,10 +1143,12 @@ MixShape mix_shape(const PassGeom& g, size_t elem) {
 }
 
 // Waves of resident tiles times a tile's time: rounds of loads, then the sums,
-// the longer of a warp's own chain (120 / 60 cycles a step with kDirectJ / one
-// output pair a thread) and the issue slots of the warps that share a
-// scheduler (34 a step for complex64, 45 for complex128 with its half-rate
-// FP64 pipe; 12 / 14 for one).
+// the longer of a warp's own chain and the issue slots of the warps that share
+// a scheduler.  Cycles a step: with kDirectJ output pairs a thread a chain of
+// 150 (complex64) or 120 and 34 / 45 slots (the FP64 pipe is half rate), with
+// one output pair 60 and 12 / 14.  The complex64 chain is what chooses best
+// over passes of 17 to 362 points (a tile alone on an SM takes 230; 120 gave
+// 353 x 8 one tile of 8 columns, 18.8 us, where four of 2 take 10.7).
 MixShape direct_shape(const PassGeom& g, size_t elem) {
   MixShape best{32, -1, 1};
   for (const int j : {kDirectJ, 1}) {
@@ -1160,7 +1162,7 @@ MixShape direct_shape(const PassGeom& g, size_t elem) {
       const int ctas = std::max(1, std::min({fit, 65536 / (nt * 80), 32}));
       const double rounds = std::ceil((double)items / nt);
       const double busy = std::min(items, nt) / 128.0;  // warps a scheduler has of one tile
-      const double chain = j == 1 ? 60.0 : 120.0;
+      const double chain = j == 1 ? 60.0 : elem == 8 ? 150.0 : 120.0;
       const double issue = j == 1 ? (elem == 8 ? 12.0 : 14.0) : (elem == 8 ? 34.0 : 45.0);
       auto wave = [&](double c) {
         const double load = 700.0 * std::ceil((double)pairs * g.W / (2 * nt)) + 0.1 * c * g.L * g.W;

@@ -71,3 +71,11 @@ def test_complex128_axes_of_many_rows_take_two_passes(dims, factors):
 def test_complex128_convolution_of_2p16():
     steps = _sm100.plan_query([22651], 1)["steps"]
     assert [s["L"] for s in steps if s["kind"] == "pass"] == [128, 512] * 2
+
+
+@pytest.mark.parametrize("dims,L,tiles", [((353, 8), 353, 4), ((17, 277), 277, 9), ((6, 314), 314, 3),
+                                          ((288, 269), 269, 144), ((337, 19, 13), 337, 124)])
+def test_few_direct_columns_are_spread_over_tiles(dims, L, tiles):
+    """complex64 direct-DFT passes of few columns: narrow tiles, so that more SMs share them."""
+    steps = [s for s in _sm100.plan_query(list(dims), 0)["steps"] if s["L"] == L]
+    assert len(steps) == 1 and steps[0]["tiles"] >= tiles, steps
