@@ -15,8 +15,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dims", [(64, 64, 32), (60, 50, 18), (97, 8)], ids=["specialised", "generic", "direct"])
 def test_refused_launch_leaves_no_error_behind(dims):
     """A capture that was already invalidated (here by a query of the capturing
-    stream) refuses the launches of an execute; the batch built afterwards
-    checks its own launch and must not meet that error."""
+    stream) refuses the launches of an execute; the plan and the batch built
+    afterwards check their own launches and must not meet that error."""
     cu = ctypes.CDLL("libcuda.so.1")
     x = o.uniform_input(dims, seed=5, dtype=np.complex64)
     a, b = S.DeviceBuffer(x.size), S.DeviceBuffer(x.size)
@@ -30,6 +30,7 @@ def test_refused_launch_leaves_no_error_behind(dims):
         plan.execute(a.ptr, b.ptr, 0, 1.0, stream.value)
     assert cu.cuStreamEndCapture(stream, ctypes.byref(graph)) != 0
     assert cu.cuStreamDestroy_v2(stream) == 0
+    _sm100.Plan((1009,)).destroy()
     batch = _sm100.Batch([dims])
     batch.execute([a.ptr], [b.ptr])
     batch.status()
