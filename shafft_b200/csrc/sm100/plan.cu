@@ -287,7 +287,7 @@ struct Planner {
       const double dear = row >= 128 ? 1.0 : row >= 64 ? 1.3 : row >= 32 ? 2.0 : 3.2;
       const double sm_bytes = std::ceil(g.ntiles / 148.0) * g.L * w * elem;
       t += sm_bytes * (direct ? 0.02 : 1.2e-4) * 0.5 * ((rows_in ? 1.0 : dear) + (rows_out ? 1.0 : dear));
-      if (least < 0 || t < least * (direct ? 0.85 : 0.92)) {
+      if (least < 0 || t < least * (direct ? 0.87 : 0.92)) {
         least = t;
         best = w;
       }
@@ -1145,7 +1145,7 @@ MixShape mix_shape(const PassGeom& g, size_t elem) {
 // Waves of resident tiles times a tile's time: rounds of loads, then the sums,
 // the longer of a warp's own chain and the issue slots of the warps that share
 // a scheduler.  Cycles a step: with kDirectJ output pairs a thread a chain of
-// 150 (complex64) or 120 and 34 / 45 slots (the FP64 pipe is half rate), with
+// 140 (complex64) or 120 and 34 / 45 slots (the FP64 pipe is half rate), with
 // one output pair 60 and 12 / 14.  The complex64 chain is what chooses best
 // over passes of 17 to 362 points (a tile alone on an SM takes 230; 120 gave
 // 353 x 8 one tile of 8 columns, 18.8 us, where four of 2 take 10.7).
@@ -1162,7 +1162,7 @@ MixShape direct_shape(const PassGeom& g, size_t elem) {
       const int ctas = std::max(1, std::min({fit, 65536 / (nt * 80), 32}));
       const double rounds = std::ceil((double)items / nt);
       const double busy = std::min(items, nt) / 128.0;  // warps a scheduler has of one tile
-      const double chain = j == 1 ? 60.0 : elem == 8 ? 150.0 : 120.0;
+      const double chain = j == 1 ? 60.0 : elem == 8 ? 140.0 : 120.0;
       const double issue = j == 1 ? (elem == 8 ? 12.0 : 14.0) : (elem == 8 ? 34.0 : 45.0);
       auto wave = [&](double c) {
         const double load = 700.0 * std::ceil((double)pairs * g.W / (2 * nt)) + 0.1 * c * g.L * g.W;
