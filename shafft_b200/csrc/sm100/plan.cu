@@ -1114,7 +1114,11 @@ RadixPlan radix_plan(int L) {
 // time: waves of resident tiles (shared memory; 768 threads an SM at 80
 // registers), a part wave counting as at least half of one, times the points
 // a busy thread handles in a tile plus the tile's own latency (first loads
-// and barriers, about six points' worth).  Measured on B200, 384^3 complex64
+// and barriers, about six points' worth).  Where all tiles are resident at
+// once a tile hardly waits for others: a part wave is then 0.7 of a full one
+// and up (one weight of at least half took 128 threads for 344 tiles of 1287 x
+// 4 complex64, 31.7 us, 256 threads 21.5; 172 tiles of 875 x 8, 21.4, for 344
+// of 875 x 4, 15.6).  Measured on B200, 384^3 complex64
 // column passes (48 KiB tiles, four CTAs): 192 threads 184 us, 128 (no idle
 // slot, but 512 threads resident) 207, 256 (a quarter idle) 207; 1225 x 1215
 // complex128 rows: 128 threads (one wave) 22.7 us, 192 (1.03 waves) 23.9.
@@ -1133,9 +1137,10 @@ MixShape mix_shape(const PassGeom& g, size_t elem) {
     }
     const double busy = slots > 0 ? nt * work / slots : nt;
     const double waves = (double)g.ntiles / (148.0 * ctas);
-    const double rest = std::ceil((waves - std::floor(waves)) * ctas - 1e-9) / ctas;
-    const double t =
-        (std::floor(waves) + (rest > 0 ? std::max(0.5, rest) : 0.0)) * ((double)g.L * g.W / busy + 6.0) *
+    const double full = std::floor(waves);
+    const double rest = std::ceil((waves - full) * ctas - 1e-9) / ctas;
+    const double part = rest <= 0 ? 0.0 : full > 0 ? std::max(0.5, rest) : 0.7 + 0.3 * rest;
+    const double t = (full + part) * ((double)g.L * g.W / busy + 6.0) *
         ((size_t)std::min<int64_t>(ctas, (g.ntiles + 147) / 148) * (smem + 1024) > (196 << 10) ? 1.2 : 1.0);
     if (best.time < 0 || t < best.time * 0.999) best = MixShape{nt, t};
   }
@@ -1505,7 +1510,7 @@ std::string describe_steps(int precision, const std::vector<Step>& steps, int64_
                   std::to_string(total) + ",\"steps\":[";
   for (size_t i = 0; i < steps.size(); ++i) {
     const Step& st = steps[i];
-    char b[768];
+    char b[800];
     if (st.kind == ST_PLANE && st.cluster) {
       snprintf(b, sizeof(b),
                "{\"kind\":\"plane\",\"L\":%d,\"planes\":%lld,\"cluster\":16,\"in\":\"%s\",\"out\":\"%s\",\"smem\":%zu}",
@@ -1520,11 +1525,11 @@ std::string describe_steps(int precision, const std::vector<Step>& steps, int64_
       for (int r = 0; r < st.g.nst; ++r) rad += (r ? "," : "") + std::to_string(st.g.rad[r]);
       snprintf(b, sizeof(b),
                "{\"kind\":\"pass\",\"L\":%d,\"radices\":[%s],\"W\":%d,\"in\":\"%s\",\"out\":\"%s\","
-               "\"in_row\":%d,\"out_row\":%d,\"tiles\":%lld,\"smem\":%zu,\"twiddle\":%d,"
+               "\"in_row\":%d,\"out_row\":%d,\"tiles\":%lld,\"threads\":%d,\"smem\":%zu,\"twiddle\":%d,"
                "\"ext\":[%lld,%lld,%lld,%lld],\"sn_in\":%lld,\"sk_out\":%lld,\"fast\":%d,\"tc\":%d,\"bs\":%d,"
                "\"map\":%d,\"prefetch\":%d}",
                st.g.L, rad.c_str(), st.g.W, buf_name(st.in_buf), buf_name(st.out_buf), st.g.in_row,
-               st.g.out_row, (long long)st.g.ntiles, st.smem, st.g.tw_mode, (long long)st.g.ext[0],
+               st.g.out_row, (long long)st.g.ntiles, st.fast || st.tc ? 0 : st.g.threads, st.smem, st.g.tw_mode, (long long)st.g.ext[0],
                (long long)st.g.ext[1], (long long)st.g.ext[2], (long long)st.g.ext[3],
                (long long)st.g.sn_in, (long long)st.g.sk_out, st.fast, st.tc, st.g.bs_mode, st.g.map_mode,
                pass_prefetch(precision, st));

@@ -79,3 +79,12 @@ def test_few_direct_columns_are_spread_over_tiles(dims, L, tiles):
     """complex64 direct-DFT passes of few columns: narrow tiles, so that more SMs share them."""
     steps = [s for s in _sm100.plan_query(list(dims), 0)["steps"] if s["L"] == L]
     assert len(steps) == 1 and steps[0]["tiles"] >= tiles, steps
+
+
+@pytest.mark.parametrize("n,L,tiles,threads", [(1769625, 1287, 344, 256), (1279395, 1053, 304, 256),
+                                               (1203125, 875, 344, 256), (1087515, 845, 322, 192)])
+def test_resident_tiles_take_large_blocks(n, L, tiles, threads):
+    """Generic complex64 passes whose tiles are all resident at once: many
+    threads a tile, and narrow tiles, rather than few tiles of few threads."""
+    step = next(s for s in _sm100.plan_query([n], 0)["steps"] if s["L"] == L)
+    assert step["tiles"] >= tiles and step["threads"] >= threads, step
