@@ -279,10 +279,13 @@ struct LenTab {
   size_t off_tw, off_p2k, off_k2p;
 };
 
-// complex64: six CTAs of 128 threads and 4096-point tiles, or three of 256
-// where a long axis needs a larger tile (the choice is made once a batch): 512
-// uneven transforms take 3.21 ms in the first form, 3.49 in the second with
-// 8192-point tiles, 3.40 as four CTAs of 192, 3.65 as twelve of 64 (B200).
+// complex64: six CTAs of 128 threads and 4096-point tiles, or three of 256 and
+// 8192-point ones where a long axis needs a larger tile (the choice is made
+// once a batch): 512 uneven transforms take 3.21 ms in the first form, 3.49 in
+// the second, 3.40 as four CTAs of 192, 3.65 as twelve of 64 (B200).  The
+// second form with 4096-point tiles is slower, long columns then have rows of
+// 16 bytes: 24 transforms with a row of 1000 to 4096 points 135 us, 126 with
+// 8192, 16 x 256 x 4096 275 and 232.
 // complex128: three CTAs of 128 threads, as many as 168 registers leave room
 // for; every axis fits.  Against tiles of half the size and, from 2358 points
 // on, one CTA of 256: 64 x 96^3 1.63 -> 1.14 ms, 8 x 2048^2 1.35 -> 1.12, 16 x
@@ -293,7 +296,7 @@ BatchForm batch_form(const std::vector<int64_t>& dims) {
   if (es == 16) return BatchForm{128, 3, 4096};
   const BatchForm form{128, 6, 4096};
   for (const int64_t L : dims)
-    if (!form.fits(2 * L * es)) return BatchForm{kThreads, 3, 4096};  // narrowest tile of a radix pass
+    if (!form.fits(2 * L * es)) return BatchForm{kThreads, 3, 8192};  // narrowest tile of a radix pass
   return form;
 }
 

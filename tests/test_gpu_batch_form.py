@@ -15,6 +15,9 @@ CASES = [
     ([(256, 4096)], S.Z2Z, 128, 256 + 256),
     ([(4096, 64)], S.Z2Z, 128, 64 + 64),
     ([(61, 128)], S.Z2Z, 128, 2 + 4),
+    # complex64: six CTAs of 128 and 4096-point tiles, or three of 256 and 8192 with a long axis
+    ([(64, 96)], S.C2C, 128, 2 + 2),
+    ([(4096, 64)], S.C2C, 256, 32 + 32),
 ]
 
 
