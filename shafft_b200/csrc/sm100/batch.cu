@@ -307,6 +307,26 @@ int64_t axis_tile(const BatchForm& form, bool direct, size_t es) {
   return direct && es == 16 ? form.tile / 2 : form.tile;
 }
 
+void digit_tables_host(int L, std::vector<uint16_t>& p2k, std::vector<uint16_t>& k2p) {
+  RadixPlan rp = radix_plan(L);
+  p2k.assign(L, 0);
+  k2p.assign(L, 0);
+  if (rp.n <= 0) return;
+  for (int p = 0; p < L; ++p) {
+    int rem = p, k = 0, pre = 1, span = L;
+    for (int s = 0; s < rp.n; ++s) {
+      const int m = span / rp.r[s];
+      const int d = rem / m;
+      rem -= d * m;
+      k += d * pre;
+      pre *= rp.r[s];
+      span = m;
+    }
+    p2k[p] = (uint16_t)k;
+    k2p[k] = (uint16_t)p;
+  }
+}
+
 template <typename T>
 int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, const BatchForm& form, int64_t tile,
                int autotune) {
@@ -350,7 +370,11 @@ int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, cons
   tb.twL = tw;
   tb.p2k = dg;
   tb.k2p = dg + L;
-  cudaMemset(dg, 0, 4 * L);
+  // the pass finds the places of its outputs through these
+  std::vector<uint16_t> p2k, k2p;
+  digit_tables_host((int)L, p2k, k2p);
+  cudaMemcpy(dg, p2k.data(), 2 * L, cudaMemcpyHostToDevice);
+  cudaMemcpy(dg + L, k2p.data(), 2 * L, cudaMemcpyHostToDevice);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -414,26 +438,6 @@ int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, cons
   cudaFree(dg);
   tune_store(key, best);
   return best;
-}
-
-void digit_tables_host(int L, std::vector<uint16_t>& p2k, std::vector<uint16_t>& k2p) {
-  RadixPlan rp = radix_plan(L);
-  p2k.assign(L, 0);
-  k2p.assign(L, 0);
-  if (rp.n <= 0) return;
-  for (int p = 0; p < L; ++p) {
-    int rem = p, k = 0, pre = 1, span = L;
-    for (int s = 0; s < rp.n; ++s) {
-      const int m = span / rp.r[s];
-      const int d = rem / m;
-      rem -= d * m;
-      k += d * pre;
-      pre *= rp.r[s];
-      span = m;
-    }
-    p2k[p] = (uint16_t)k;
-    k2p[k] = (uint16_t)p;
-  }
 }
 
 template <typename T>
