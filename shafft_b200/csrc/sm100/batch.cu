@@ -328,17 +328,17 @@ void digit_tables_host(int L, std::vector<uint16_t>& p2k, std::vector<uint16_t>&
 }
 
 template <typename T>
-int tune_width(int64_t L, bool row, int64_t ext0, int default_w, size_t es, const BatchForm& form, int64_t tile,
+int tune_width(int64_t L, bool row, int default_w, size_t es, const BatchForm& form, int64_t tile,
                int autotune) {
   const int maxw_smem = (int)std::max<int64_t>(1, (96 * 1024) / ((L + 1) * (int64_t)es));
   std::vector<int> cands;
   // tiles of a quarter of `tile` to `tile` points, 256 rows or 64 columns (the
-  // width of the synthetic column tensor) at most
+  // width of the synthetic column tensor) at most; whatever the batch
+  // dimension of the axis at hand, since the answer serves all of that length
   const int wmax = row ? kBatchRowWMax : kBatchColWMax;
   for (int w = 1; w <= wmax; w *= 2) {
     if (w > maxw_smem || (w > 1 && (int64_t)w * L > tile)) break;
-    if ((int64_t)w * L * 4 < tile && w < wmax && w < ext0) continue;
-    if (w > 1 && w / 2 >= ext0) break;
+    if ((int64_t)w * L * 4 < tile && w < wmax) continue;
     cands.push_back(w);
   }
   if (cands.empty()) return default_w;
@@ -491,14 +491,14 @@ int batch_build(shafft_sm100_batch_s* b, int autotune) {
       if (row) {
         // tile widths are powers of two (the tile walks columns by mask and shift)
         const int def = pow2_floor((int)std::min<int64_t>(kBatchRowWDefault, std::max<int64_t>(1, tile / L)));
-        W = tune_width<T>(L, true, O, def, es, form, tile, autotune);
+        W = tune_width<T>(L, true, def, es, form, tile, autotune);
         g.ext[0] = O;
         g.sin[0] = g.sout[0] = L;
         g.ext[1] = g.ext[2] = g.ext[3] = 1;
         g.sn_in = g.sk_out = 1;
       } else {
         const int def = pow2_floor((int)std::min<int64_t>(kBatchColWDefault, std::max<int64_t>(1, tile / L)));
-        W = tune_width<T>(L, false, I, def, es, form, tile, autotune);
+        W = tune_width<T>(L, false, def, es, form, tile, autotune);
         g.ext[0] = I;
         g.sin[0] = g.sout[0] = 1;
         g.ext[1] = O;
