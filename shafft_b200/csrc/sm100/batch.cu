@@ -200,6 +200,10 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1)
 // ---------------------------------------------------------------------------
 // autotuner cache
 // ---------------------------------------------------------------------------
+// Part of every key: counted up when the kernel or the tuner changes, so that
+// widths measured before are not used (entries without one are of the kernel
+// with per-element shared accesses).
+constexpr int kTuneRevision = 2;
 std::mutex g_tune_mu;
 std::map<std::string, int> g_tune;
 bool g_tune_loaded = false;
@@ -342,8 +346,11 @@ int tune_width(int64_t L, bool row, int default_w, size_t es, const BatchForm& f
     cands.push_back(w);
   }
   if (cands.empty()) return default_w;
+  // what the width was measured on: the kernel's revision (kTuneRevision) and
+  // the shape the batch launches it with
   const std::string key = std::string(es == 8 ? "c64" : "c128") + ":L=" + std::to_string(L) +
-                          (row ? ":row" : ":col");
+                          (row ? ":row" : ":col") + ":r" + std::to_string(kTuneRevision) + ":t" +
+                          std::to_string(form.threads);
   std::lock_guard<std::mutex> lk(g_tune_mu);
   tune_load();
   auto it = g_tune.find(key);

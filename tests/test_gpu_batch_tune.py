@@ -30,3 +30,19 @@ def test_width_does_not_depend_on_the_batch_dimension_it_was_met_with(tmp_path):
     _run("from shafft_b200 import _sm100; _sm100.Batch([(16, 2)], 0, autotune=True)", cache)
     w = {k: int(v) for k, v in _widths(cache).items() if k.startswith("c64:L=16:col")}
     assert len(w) == 1 and min(w.values()) >= 64, w
+
+
+def test_widths_of_another_kernel_revision_are_not_used(tmp_path):
+    """Entries without the revision (those of the kernel before) and of another
+    one leave the default widths in place; an entry of this one is used."""
+    code = "from shafft_b200 import _sm100; print(_sm100.Batch([(64, 96)], 0).describe()['tiles'])"
+    none = int(_run(code, tmp_path / "none.txt"))
+    old = tmp_path / "old.txt"
+    old.write_text("c64:L=96:row 2\nc64:L=64:col 2\nc64:L=96:row:r1:t128 2\nc64:L=64:col:r1:t128 2\n")
+    assert int(_run(code, old)) == none
+    tuned = tmp_path / "tuned.txt"
+    _run("from shafft_b200 import _sm100; _sm100.Batch([(64, 96)], 0, autotune=True)", tuned)
+    keys = [k for k in _widths(tuned) if k.startswith("c64:L=96:row")]
+    assert len(keys) == 1
+    tuned.write_text(f"{keys[0]} 2\n")
+    assert int(_run(code, tuned)) > none
