@@ -3,7 +3,7 @@
 //
 // k_fft_direct -- one HBM pass of batched length-L DFTs on W-wide tiles for
 // lengths with a prime factor above 13: the tile is loaded in natural order
-// and every output is an O(L) sum, evaluated in pairs (direct_store).
+// and every output is an O(L) sum, evaluated in pairs (direct_sums).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -365,7 +365,10 @@ __device__ __forceinline__ void mix_tile(const PassGeom& g, const typename Cx<T>
 #undef SHAFFT_CALL
 }
 
-// 256 threads x 3 CTAs per SM: at most 85 registers
+// 256 threads x 3 CTAs per SM, i.e. at most 85 registers; every instance is
+// compiled to 80.  The radix 11 and 13 stages of a chunk need more, and spill:
+// 104 bytes a thread (complex64 unpermuted), 60 (permuted), 188 and 268
+// (complex128); the one-column complex64 instance does not.
 template <typename T, int VW, bool SWZ>
 __global__ void __launch_bounds__(kThreads, 3)
     k_fft_mix(const __grid_constant__ PassGeom g, const typename Cx<T>::type* in, typename Cx<T>::type* out,

@@ -14,9 +14,8 @@
 // consecutive elements when sn_in/sk_out == 1 ("row" orientation).
 //
 // Optional extras fused into the same pass:
-//   * a four-step twiddle  w_N^{(n or k) * t}  with t = b_{tw_dim} (applied to
-//     the input (PRE) or to the output (POST)); the planner guarantees the
-//     exponent is < N so no modular reduction is needed;
+//   * a four-step twiddle  w_N^{k * t}  with t = b_{tw_dim} on the output; the
+//     planner guarantees the exponent is < N so no modular reduction is needed;
 //   * conjugation on input / output (backward transforms are computed as
 //     conj(F(conj(x))));
 //   * a real scale on output (fused normalisation).
@@ -29,7 +28,7 @@ constexpr int kMaxStages = 8;
 constexpr int kMaxPassLen = 4096;
 constexpr int kThreads = 256;
 
-enum TwMode : int { TW_NONE = 0, TW_PRE = 1, TW_POST = 2 };
+enum TwMode : int { TW_NONE = 0, TW_POST = 2 };
 
 struct RadixPlan {
   int n = 0;
@@ -55,7 +54,7 @@ struct alignas(16) PassGeom {
   int vec_in, vec_out;        // complex64: two neighbouring columns are one aligned 16-byte vector
   int W;       // tile width along b0 (power of two)
   int logW;
-  int pitch;   // shared-memory row pitch in elements: element (p, w) at p*pitch + w
+  int pitch;   // shared-memory row pitch in elements (generic_pitch): direct DFT: element (p, w) at p*pitch + w
   int in_row;  // 1: lanes walk n at load (sn_in == 1)
   int out_row; // 1: lanes walk k at store (sk_out == 1)
   int64_t ext[4];
@@ -65,7 +64,8 @@ struct alignas(16) PassGeom {
   int64_t tiles_w;  // ceil(ext[0] / W)
   int64_t ntiles;   // tiles_w * ext[1] * ext[2] * ext[3]
   // division of a tile index < 2^31 by d = tiles_w, ext[1], ext[2]:
-  // (umulhi(x, mul) + x) >> sh (tile_idx)
+  // (umulhi(x, mul) + x) >> sh (tile_idx), with mul and sh as in Granlund and
+  // Montgomery, "Division by Invariant Integers using Multiplication" (1994)
   uint32_t tdiv_mul[3];
   uint32_t tdiv_sh[3];
   int tw_mode;
@@ -163,16 +163,15 @@ __device__ __forceinline__ TileIdx tile_idx(const PassGeom& g, int64_t tile) {
 enum BsMode : int { BS_LOAD_MOD = 1, BS_STORE_MULH = 2, BS_STORE_DEMOD = 4 };
 enum MapMode : int { MAP_LOAD = 1, MAP_STORE = 2 };
 
-// Shared-memory row pitch (elements) of a generic-pass tile [L][pitch] whose
-// rows hold W columns.  Column-input passes put the W columns of a row on
-// consecutive lanes, so a pitch of W keeps their half-warps of 8-byte
-// accesses on distinct banks.  Row-input passes put consecutive rows on
-// consecutive lanes: with W >= 8 a pitch of W would put a half-warp on one
-// bank pair, so they get the odd pitch W + 1; with W <= 4 the conflict is at
-// most 4-way and the smaller tile wins.  Measured on B200 against W + 1
-// everywhere, FFT1D 1,488,375 fwd+bwd (W = 4): complex64 0.091 -> 0.083 ms,
-// complex128 0.152 -> 0.115 ms, the batched form unchanged; W everywhere
-// cost the batched form (row passes up to W = 32) 3%.
+// Shared-memory row pitch (elements) of a generic or direct-DFT tile
+// [L][pitch] whose rows hold W columns.  Direct-DFT passes address the tile by
+// it: column-input ones put the W columns of a row on consecutive lanes, so a
+// pitch of W keeps their half-warps of 8-byte accesses on distinct banks;
+// row-input ones put consecutive rows on consecutive lanes, where with W >= 8
+// a pitch of W would put a half-warp on one bank pair, so they get the odd
+// pitch W + 1.  Radix passes (k_fft_mix) permute 16-byte chunks instead and
+// use L * W elements of the tile; their row tiles of W >= 8 are still sized by
+// this rule, one part in W more than they need.
 __host__ __device__ constexpr int generic_pitch(int W, bool in_row) {
   return W == 1 ? 1 : ((in_row && W >= 8) ? W + 1 : W);
 }

@@ -99,7 +99,7 @@ struct Step {
   int in_buf = BUF_SRC, out_buf = BUF_DST;
   int tabL = -1, tabN = -1, tabB = -1;
   int64_t bsL = 0, bsM = 0, bsI = 1, total = 0;
-  size_t smem = 0;
+  size_t smem = 0;   // bytes of the tile; a launch may ask for more (pass_smem: direct-DFT twiddles)
   int fast = 0;      // 1: specialised k_fft_fast pass (compile-time L)
   int fast_row = 0;  // specialised pass reads row tiles (transposing)
   int tc = 0;        // 1: tensor-core pass (tcgen05 split-FP16 DFT GEMM, L <= 64)
@@ -247,7 +247,7 @@ struct Planner {
   void try_fast(Step& st) {
     if (cur_tc) return mark_tc(st);
     PassGeom& g = st.g;
-    if (!fast_len(g.L) || g.tw_mode == TW_PRE) return;
+    if (!fast_len(g.L)) return;
     const bool in_row = (g.sn_in == 1);
     if (!fast_geom(g, in_row)) return;
     if (in_row && st.in_buf == st.out_buf) return;  // transposing pass must be out of place

@@ -290,8 +290,6 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       for (int j = 0; j < 8; ++j) {
         float2 x = v[i][j];
         if (g.conj_in) x.y = -x.y;
-        if (g.tw_mode == TW_PRE && R.in[r] >= 0 && 8 * c + j < L)
-          x = cmul(x, tw_n(tb, g.tw_shift, g.tw_mask, (int64_t)(8 * c + j) * R.t[r]));
         v[i][j] = x;
         mx = fmaxf(mx, fmaxf(fabsf(x.x), fabsf(x.y)));
       }
