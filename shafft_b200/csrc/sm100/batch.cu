@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1)
 // Part of every key: counted up when the kernel or the tuner changes, so that
 // widths measured before are not used (entries without one are of the kernel
 // with per-element shared accesses).
-constexpr int kTuneRevision = 2;
+constexpr int kTuneRevision = 3;
 std::mutex g_tune_mu;
 std::map<std::string, int> g_tune;
 bool g_tune_loaded = false;
@@ -430,8 +430,12 @@ int tune_width(int64_t L, bool row, int default_w, size_t es, const BatchForm& f
     }
     if (cudaGetLastError() != cudaSuccess || launched != cudaSuccess) continue;
     // in a batch each tile also costs its CTA a ticket (atomic, slot lookup,
-    // wait, geometry: about 2 us), which this launch does without
-    ms += 3 * 2e-3f * (float)g.ntiles / (148 * form.ctas);
+    // wait for the previous pass, geometry) with the CTA's other warps idle,
+    // which this launch does without: 16 us, fitted on batches tuned with it
+    // (B200, 4096 uneven complex64 transforms 28.4 ms with 2 us, 25.6 with 8,
+    // 25.5 with 16, 25.8 with 40, the default widths; 128 complex128 ones 1.80,
+    // 1.51, 1.46, 1.45)
+    ms += 3 * 16e-3f * (float)g.ntiles / (148 * form.ctas);
     if (ms < best_ms) {
       best_ms = ms;
       best = w;
