@@ -107,7 +107,6 @@ __global__ void __launch_bounds__(256)
   const C* zm = Z + mr * H;
   C* xr = X + r * (H + 1);
   C* xm = X + mr * (H + 1);
-  const T half = (T)0.5 * scale;
   C a[kRcUnroll], b[kRcUnroll], w[kRcUnroll];
 #pragma unroll
   for (int u = 0; u < kRcUnroll; ++u) {
@@ -121,10 +120,11 @@ __global__ void __launch_bounds__(256)
   for (int u = 0; u < kRcUnroll; ++u) {
     const int64_t k = k0 + ((int64_t)u << logG);
     if (k >= H) continue;
-    const C e = C{(a[u].x + b[u].x) * half, (a[u].y - b[u].y) * half};
+    const C e = C{(a[u].x + b[u].x) * (T)0.5, (a[u].y - b[u].y) * (T)0.5};
     // (a - conj(z)) / (2i) = (a.y + z.y, -(a.x - z.x)) / 2
-    const C o = cmul(C{(a[u].y + b[u].y) * half, (b[u].x - a[u].x) * half}, w[u]);
-    const C p = cadd(e, o), q = cconj(csub(e, o));
+    const C o = cmul(C{(a[u].y + b[u].y) * (T)0.5, (b[u].x - a[u].x) * (T)0.5}, w[u]);
+    // the scale last: one more rounding of the finished value, none inside
+    const C p = cscale(cadd(e, o), scale), q = cscale(cconj(csub(e, o)), scale);
     xr[k] = p;
     if (k == 0) xr[H] = cconj(q);  // Z[J, H] is Z[J, 0] and w^H = -1
     if (r != mr) {
