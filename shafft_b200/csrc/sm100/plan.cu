@@ -519,7 +519,9 @@ struct Planner {
     // larger last factor): three passes over tiles that leave room for several
     // CTAs per SM beat two over 64 and 128 KiB tiles.  B200, device time, two
     // and three factors: complex64 2^17 256*512 10.2 / 10.7 us, 2^19 512*1024
-    // 16.1 / 64*64*128 11.8, 2^20 1024*1024 19.9 / 64*64*256 14.4.  Between
+    // 16.1 / 64*64*128 11.8, 2^20 1024*1024 19.9 / 64*64*256 14.4, with one
+    // twiddle more (relative error of 2^19 1.7e-7 / 2.0e-7, as 2^21; of its
+    // convolutions 3.1e-7 / 4.0e-7; complex128 unchanged).  Between
     // 2^16 and 2^18 complex128 takes three only where the whole tensor is too
     // small for two to fill the chip: 2^17 256*512 / 32*32*128 alone 11.6 / 9.6,
     // twice 22.2 / 21.1, 4 times 23.4 / 24.4, 64 times 168 / 183.  (2^18 stays
